@@ -9,6 +9,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -86,6 +87,8 @@ struct BoltCtx {
     double* es_part;
     double2 *es_rho, *es_e;
     int es_fwd, es_inv;
+    double* es_green;       // N_q2 = 1: Green's function of the periodic solve [N_q1]
+    const double* es_density;   // ... and the density sums the next p-stage solves with
     // block neighbours' copies of (f, buf[0], buf[1]): [0] below, [1] above
     // (q2), [2] left, [3] right (q1); peer_on bit 1: q2 on, bit 2: q1 on
     void* peer[4][3];
@@ -118,6 +121,7 @@ struct BoltCtx {
     double timing_ms[BOLT_TIMING_COUNT];
     int timing_on, timing_depth;
     int pair_enabled;       // paired kernel allowed (BOLT_NO_PAIR unset)
+    PShape pshape;          // launch shape of the p-stage kernel
     int pair_shape_ok;      // grid/method meet the paired kernel's shape conditions
 };
 
@@ -192,6 +196,32 @@ static const CUtensorMap* get_tmap(BoltCtx* ctx, const void* ptr, int kind) {
     ctx->tmaps[slot].kind = kind;
     ctx->tmaps[slot].map = m;
     return &ctx->tmaps[slot].map;
+}
+
+// Green's function of the electrostatic solve on a periodic line of n cells
+// (fft.py:9-78 with one q2 cell): E = real(ifft(-i rho_hat / (2 pi k))), k = 0 left
+// out, is sum_j G_{i-j} rho_j with G_m = (1/n) sum_{k=1}^{(n-1)/2} sin(2 pi k m / n)
+// / (pi k / (n dq)); the Nyquist mode of an even n is imaginary and drops out.
+// Up to kGreenMax cells: every p-stage CTA reads n of its values (16 KB), which
+// costs less than the solve's launches; longer lines use the FFT.
+constexpr int kGreenMax = 2048;
+
+static std::vector<double> line_green(int n, double dq) {
+    const long double pi = 3.14159265358979323846264338327950288L;
+    std::vector<long double> sn(n);
+    for (int j = 0; j < n; ++j) sn[j] = sinl(2 * pi * j / n);
+    std::vector<double> G(n);
+    for (int m = 0; m < n; ++m) {
+        long double v = 0;
+        long long km = 0;
+        for (int k = 1; k <= (n - 1) / 2; ++k) {
+            km += m;
+            if (km >= n) km -= n;
+            v += sn[km] / k;
+        }
+        G[m] = (double)(v * (long double)dq / pi);
+    }
+    return G;
 }
 
 extern "C" {
@@ -292,6 +322,9 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
     const size_t rowbytes = (size_t)g.N_s * ctx->Np * ctx->elem;
     ctx->use_tma_ok = (g.N_ghost >= HALO) && (rowbytes % 16 == 0) &&
                       (((size_t)ctx->Np * ctx->elem) % 16 == 0) && get_encode_fn() != nullptr;
+    if (p.fields_enabled)
+        ctx->pshape = choose_pshape(g.N_p1, g.N_p2, g.N_p3, ctx->elem,
+                                    (long long)g.N_q1 * g.N_q2 * g.N_s, current_sm_count());
     ctx->at_n = 1;
     ctx->pair_enabled = getenv("BOLT_NO_PAIR") == nullptr;
 
@@ -320,7 +353,14 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
             rc = dev_alloc(ctx, (void**)&ctx->es_part, kNumMom * plane * sizeof(double));
             if (rc == BOLT_OK) rc = dev_alloc(ctx, (void**)&ctx->es_rho, nq * sizeof(double2));
             if (rc == BOLT_OK) rc = dev_alloc(ctx, (void**)&ctx->es_e, 2 * nq * sizeof(double2));
-            if (rc == BOLT_OK && poisson_plans_create(g.N_q1, g.N_q2, &ctx->es_fwd, &ctx->es_inv))
+            if (rc == BOLT_OK && g.N_q2 == 1 && g.N_q1 <= kGreenMax) {
+                const std::vector<double> G = line_green(g.N_q1, g.dq1);
+                rc = dev_alloc(ctx, (void**)&ctx->es_green, G.size() * sizeof(double));
+                if (rc == BOLT_OK && cudaMemcpy(ctx->es_green, G.data(),
+                                                G.size() * sizeof(double),
+                                                cudaMemcpyHostToDevice) != cudaSuccess)
+                    rc = BOLT_ERR_CUDA;
+            } else if (rc == BOLT_OK && poisson_plans_create(g.N_q1, g.N_q2, &ctx->es_fwd, &ctx->es_inv))
                 rc = BOLT_ERR_CUDA;
         }
     }
@@ -362,6 +402,7 @@ void bolt_ctx_destroy(BoltCtx* ctx) {
     cudaFree(ctx->es_part);
     cudaFree(ctx->es_rho);
     cudaFree(ctx->es_e);
+    cudaFree(ctx->es_green);
     poisson_plans_destroy(ctx->es_fwd, ctx->es_inv);
     if (ctx->hflag) cudaFreeHost(ctx->hflag);
     if (ctx->timed) {
@@ -778,6 +819,10 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
     return BOLT_OK;
 }
 
+static int electrostatic(const BoltCtx* ctx) {
+    return ctx->p.fields_enabled && ctx->p.fields_type == BOLT_FIELDS_ELECTROSTATIC;
+}
+
 static int launch_pstage(BoltCtx* ctx, const StageIO& io, const void* kq, cudaStream_t st,
                          int term = 0) {
     TimedScope ts(ctx, BOLT_TIMING_PSTAGE, st);
@@ -807,11 +852,26 @@ static int launch_pstage(BoltCtx* ctx, const StageIO& io, const void* kq, cudaSt
         a.flag = nullptr;
     }
     a.sg = ctx->sg;
-    const size_t smem = pstage_smem(ctx->Np, ctx->elem, g.N_p1 + g.N_p2 + g.N_p3);
-    if (smem > 200 * 1024) return BOLT_ERR_UNSUPPORTED;
+    if (electrostatic(ctx) && ctx->es_green) {
+        a.green = ctx->es_green;
+        a.density = ctx->es_density;
+        a.cell_out = ctx->cell;
+        a.eps = ctx->p.eps;
+        a.mom_scale = ctx->sg.polar2d ? ctx->sg.mom_scale : 1.0;
+        for (int s = 0; s < g.N_s; ++s) a.measure[s] = (g.dp3[s] * g.dp2[s]) * g.dp1[s];
+    }
+    if (!pstage_fits(ctx->Np, ctx->elem, g.N_p1 + g.N_p2 + g.N_p3)) return BOLT_ERR_UNSUPPORTED;
+    const PShape& sh = ctx->pshape;
+    for (int ax = 0; ax < 3; ++ax) a.seg[ax] = sh.seg[ax];
+    // N_p1 a multiple of the vector keeps every q-cell's block and p1 row aligned
+    a.vec = g.N_p1 % (16 / (int)ctx->elem) == 0;
+    const void* ptrs[6] = {a.fs, a.kq, a.base1, a.base2, a.out1, a.out2};
+    for (const void* p : ptrs)
+        if ((uintptr_t)p % 16 != 0) a.vec = 0;
     dim3 grid(g.N_q1 * g.N_q2, g.N_s);
-    cudaError_t e = ctx->elem == 8 ? launch_pstage_f64(a, ctx->recon_p, grid, smem, st)
-                                   : launch_pstage_f32(a, ctx->recon_p, grid, smem, st);
+    cudaError_t e = ctx->elem == 8
+        ? launch_pstage_f64(a, ctx->recon_p, grid, sh.threads, sh.smem, st)
+        : launch_pstage_f32(a, ctx->recon_p, grid, sh.threads, sh.smem, st);
     ctx->launches++;
     CK(e);
     return BOLT_OK;
@@ -847,20 +907,24 @@ static int launch_fields(BoltCtx* ctx, double dt, int nsplit_j, cudaStream_t st,
     return BOLT_OK;
 }
 
-static int electrostatic(const BoltCtx* ctx) {
-    return ctx->p.fields_enabled && ctx->p.fields_type == BOLT_FIELDS_ELECTROSTATIC;
-}
-
 // electrostatic fields of the df/dt argument f (df_dt_fvm.py:234-242): its
 // species densities, then the FFT Poisson solve into the cell-centred E1, E2
-static int launch_electrostatic(BoltCtx* ctx, const void* f, cudaStream_t st) {
+// (part: the sums of f that the stage which wrote f left, [5][Ns][Nq2][Nq1], or
+// null: a moment pass over f); on a line (es_green) the p-stage solves for E
+static int launch_electrostatic(BoltCtx* ctx, const void* f, const double* part,
+                                cudaStream_t st) {
     TimedScope ts(ctx, BOLT_TIMING_FIELDS, st);
     const BoltGrid& g = ctx->g;
-    int rc = launch_moments5(ctx, f, ctx->es_part, st);
-    if (rc) return rc;
+    if (!part) {
+        const int rc = launch_moments5(ctx, f, ctx->es_part, st);
+        if (rc) return rc;
+        part = ctx->es_part;
+    }
+    ctx->es_density = part;
+    if (ctx->es_green) return BOLT_OK;
     PoissonArgs a;
     memset(&a, 0, sizeof(a));
-    a.part = ctx->es_part;
+    a.part = part;
     a.rho_hat = ctx->es_rho;
     a.e_hat = ctx->es_e;
     a.cell = ctx->cell;
@@ -886,7 +950,7 @@ static int run_stage(BoltCtx* ctx, StageIO io, int evolve, double dt, cudaStream
     if (!ctx->p.fields_enabled) {
         rc = launch_qstage(ctx, io, 0, 0, st, region);
     } else if (electrostatic(ctx)) {
-        rc = launch_electrostatic(ctx, io.fs, st);
+        rc = launch_electrostatic(ctx, io.fs, io.mom_in, st);
         StageIO qio = io;
         qio.out1 = ctx->kbuf;
         if (rc == BOLT_OK && ctx->p_only) {
@@ -922,7 +986,7 @@ static int ensure_state(BoltCtx* ctx, void* f, cudaStream_t st) {
         if (rc) return rc;
     }
     ctx->ghost_stale_time = 0;
-    if (ctx->bgk && ctx->mom_owner != f) {
+    if ((ctx->bgk || electrostatic(ctx)) && ctx->mom_owner != f) {
         rc = launch_moments5(ctx, f, ctx->momP[ctx->cur_mom], st);
         if (rc) return rc;
         ctx->cur_nsplit = 1;
@@ -1001,7 +1065,10 @@ static int run_rk_stage(BoltCtx* ctx, void* f, double dt, int k, cudaStream_t st
     memset(&io, 0, sizeof(io));
     io.mom_in = m_in;
     io.nsplit_in = nin;
-    io.mom_out = ctx->bgk ? m_out : nullptr;
+    // the moments of a stage's output serve the next one's Maxwellian, and its
+    // electrostatic solve
+    const bool track = ctx->bgk || electrostatic(ctx);
+    io.mom_out = track ? m_out : nullptr;
     const int last = k == stage_count(ctx) - 1;
     io.flag = last ? ctx->dflag : nullptr;
     void* out1;
@@ -1069,7 +1136,7 @@ static int run_rk_stage(BoltCtx* ctx, void* f, double dt, int k, cudaStream_t st
     if (last) {
         ctx->cur_nsplit = mo_split;
         ctx->ghost_owner = f;
-        ctx->mom_owner = ctx->bgk ? f : nullptr;
+        ctx->mom_owner = track ? f : nullptr;
     }
     return BOLT_OK;
 }
@@ -1351,7 +1418,7 @@ static int dfdt_impl(BoltCtx* ctx, const void* f_dev, void* dfdt_dev, int evolve
         return launch_qstage(ctx, io, 1, 0, st);
     }
     if (electrostatic(ctx)) {
-        rc = launch_electrostatic(ctx, f_dev, st);
+        rc = launch_electrostatic(ctx, f_dev, ctx->bgk ? m : nullptr, st);
         evolve_fields = 0;
     }
     if (rc) return rc;

@@ -183,10 +183,23 @@ struct PStageArgs {
     int Nq1, Nq2, Ng, Ns, Np1, Np2, Np3, Np, Nq1g, Nq2g;
     int periodic1, periodic2;
     int term;              // 0: the stage combine; 1..3: out1 <- d_flux_pk_dpk alone
+    int seg[3];            // pieces that each line along p1, p2, p3 is walked in
+    int vec;               // 16-byte vectors: N_p1 a multiple, every buffer aligned
+    // electrostatic fields of a q-line (N_q2 = 1): E1 of the CTA's cell from the
+    // line's densities and the Green's function of the periodic solve (null:
+    // the fields in `cell`), written to `cell_out` for the fields API
+    const double* green;   // [Nq1]
+    const double* density; // partial sums of fs [Ns][Nq1]
+    double* cell_out;
+    double eps, mom_scale, measure[kMaxSpecies];
     SpeciesGrid sg;
 };
 
-constexpr int PTHREADS = 256;
+constexpr int PTHREADS_MAX = 512;
+
+// elements from one p1 row of the p-stage's shared-memory blocks to the next:
+// odd, so that lanes walking neighbouring rows read distinct banks
+__host__ __device__ inline int pstage_pitch(int Np1) { return Np1 | 1; }
 
 struct FieldArgs {
     double* yee;            // [6][Nq2g][Nq1g]

@@ -332,6 +332,13 @@ __device__ __forceinline__ double add2(double a, double b) { return a + b; }
 __device__ __forceinline__ double sub2(double a, double b) { return a - b; }
 __device__ __forceinline__ double rcp2(double a) { return rcp_nr(a); }
 
+// one FP32 value per thread
+__device__ __forceinline__ float fma2(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float mul2(float a, float b) { return a * b; }
+__device__ __forceinline__ float add2(float a, float b) { return a + b; }
+__device__ __forceinline__ float sub2(float a, float b) { return a - b; }
+__device__ __forceinline__ float rcp2(float a) { return fast_rcp(a); }
+
 // lane value -> its element type, a constant broadcast to it, and its
 // components (n = 2 for a pair, 1 for a scalar)
 template <typename P> struct LaneOf;
@@ -345,6 +352,11 @@ template <> struct LaneOf<double2> {
     static constexpr int n = 2;
     __device__ static double2 splat(double a) { return make_double2(a, a); }
 };
+template <> struct LaneOf<float> {
+    typedef float E;
+    static constexpr int n = 1;
+    __device__ static float splat(float a) { return a; }
+};
 template <> struct LaneOf<double> {
     typedef double E;
     static constexpr int n = 1;
@@ -354,6 +366,7 @@ template <> struct LaneOf<double> {
 __device__ __forceinline__ float& comp(float2& v, int c) { return c ? v.y : v.x; }
 __device__ __forceinline__ double& comp(double2& v, int c) { return c ? v.y : v.x; }
 __device__ __forceinline__ double& comp(double& v, int) { return v; }
+__device__ __forceinline__ float& comp(float& v, int) { return v; }
 
 // element type -> pair type and the walker's constants in that type
 template <typename E> struct PairOf;
@@ -503,6 +516,33 @@ struct ConstPairWalkerT {
     __device__ __forceinline__ P next(P, P, P y2, P, P, const Side&) {
         return add2(y2, y2);
     }
+};
+
+// Face walker of one p-line: the reference-order faces in FP64, the sliding
+// third-difference form (which returns twice the face value) in FP32
+template <int RECON, bool EXACT, typename T> struct PLineWalker {
+    typedef Weno5Side<T> Side;
+    FaceWalker<RECON, EXACT, T> w;
+    __device__ __forceinline__ T first(T y0, T y1, T y2, T y3, T y4, bool right, const Side& S) {
+        return w.first(y0, y1, y2, y3, y4, right, S);
+    }
+    __device__ __forceinline__ T next(T y0, T y1, T y2, T y3, T y4, bool right, const Side& S) {
+        return w.next(y0, y1, y2, y3, y4, right, S);
+    }
+    __device__ __forceinline__ static T flux(T C, T face) { return C * face; }
+};
+template <> struct PLineWalker<BOLT_RECON_WENO5, false, float> {
+    typedef Weno5PairT<float, float> Side;
+    Weno5PairWalkerT<float, float> w;
+    __device__ __forceinline__ float first(float y0, float y1, float y2, float y3, float y4, bool,
+                                           const Side& S) {
+        return w.first(y0, y1, y2, y3, y4, S);
+    }
+    __device__ __forceinline__ float next(float y0, float y1, float y2, float y3, float y4, bool,
+                                          const Side& S) {
+        return w.next(y0, y1, y2, y3, y4, S);
+    }
+    __device__ __forceinline__ static float flux(float C, float face) { return (0.5f * C) * face; }
 };
 
 // ---------------------------------------------------------------------------

@@ -7,9 +7,10 @@
 //                   FP64 partial moments of the stage output.  This is
 //                   df_dt_fvm.py:56-97 (q-part and source) fused with the
 //                   stage update of fvm_operator.py:26,33 / integrators.py:15-28.
-//   pstage_kernel   p1/p2/p3 advection with C_p from the cell-centred fields
-//                   (df_dt_fvm.py:245-323), added to the q-part, then the RK
-//                   combine (used only when fields are enabled).
+//   pstage_kernel   (pstage_kernel.cuh) p1/p2/p3 advection with C_p from the
+//                   cell-centred fields (df_dt_fvm.py:245-323), added to the
+//                   q-part, then the RK combine (used only when fields are
+//                   enabled).
 //   moments_kernel  compute_moments.py:7-59 for any moment of moments.py.
 //   ghost_kernel    communicate_f + apply_bcs_f (periodic wrap, mirror,
 //                   Dirichlet inflow, zero for ghosted outflow cells).
@@ -566,183 +567,6 @@ qstage_kernel(const __grid_constant__ QStageArgs a) {
             if (ii < Nq1 && jj < Nq2)
                 a.j_out[(((long long)split * 3 + q) * a.Ns + s) * plane
                         + (long long)jj * Nq1 + ii] = j_acc[c];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// p-stage kernel (fields enabled): one CTA per (interior q-cell, species)
-// holds the whole p-block in shared memory.
-//   k = k_q + (-(d1 + d2 + d3)),  d_a = (F_a(right) - F_a(left)) * (1/dp_a)
-// (df_dt_fvm.py:245-323), with circular neighbours along each p axis, C_p
-// from the cell-centred fields (advection_terms.py:147-188), then the RK
-// combine and the FP64 moments of out1 (full sums: nsplit = 1).
-// ---------------------------------------------------------------------------
-
-// q / n and q % n for 0 <= q < 2^24 with n >= 1, from a float reciprocal
-// and one correction step
-struct PDiv {
-    int n;
-    float inv;
-    __device__ __forceinline__ void set(int nn) { n = nn; inv = 1.0f / float(nn); }
-    __device__ __forceinline__ int div(int q, int* rem) const {
-        int d = __float2int_rz(float(q) * inv);
-        int r = q - d * n;
-        if (r < 0) { --d; r += n; }
-        else if (r >= n) { ++d; r -= n; }
-        *rem = r;
-        return d;
-    }
-};
-
-// flux at the left face of element c along an axis with n cells (n >= 3: a
-// window position pos-3 .. pos+2 wraps at most once), pos its index along
-// the axis, neighbours circular within the axis
-template <int RECON, bool EXACT, typename T>
-__device__ __forceinline__ T p_face_flux(const T* fb, int c, int stride, int n, int pos,
-                                         T C, const Weno5Side<T>& Sr, const Weno5Side<T>& Sl) {
-    const bool right = C > T(0);
-    const int off = right ? -3 : -2;          // window start relative to the cell
-    T y[5];
-#pragma unroll
-    for (int t = 0; t < 5; ++t) {
-        int q = pos + off + t;
-        if (n >= 3) {
-            q = q < 0 ? q + n : (q >= n ? q - n : q);
-        } else {
-            q = ((q % n) + n) % n;
-        }
-        y[t] = fb[c + (q - pos) * stride];
-    }
-    T fv = face_value<RECON, EXACT>(y[0], y[1], y[2], y[3], y[4], right, right ? Sr : Sl);
-    return C * fv;
-}
-
-template <typename T, bool EXACT, int RECON>
-__global__ void __launch_bounds__(PTHREADS)
-pstage_kernel(const __grid_constant__ PStageArgs a) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    T* fb = reinterpret_cast<T*>(smem_raw);      // [Np]
-    T* Fx[3] = {fb + a.Np, fb + 2 * a.Np, fb + 3 * a.Np};   // left-face fluxes per p axis
-    // p-cell centres of the species along p1, p2, p3 (after the four arrays,
-    // 8-byte aligned)
-    double* vg = reinterpret_cast<double*>(smem_raw + ((4 * (size_t)a.Np * sizeof(T) + 7) & ~(size_t)7));
-    __shared__ double red[PTHREADS / 32][kNumMom];
-
-    const int tid = threadIdx.x;
-    const int ii = blockIdx.x % a.Nq1, jj = blockIdx.x / a.Nq1, s = blockIdx.y;
-    const long long rowstride = (long long)a.Ns * a.Np;
-    const long long colstride = rowstride * a.Nq1g;
-    const long long cbase = (long long)(jj + a.Ng) * colstride + (long long)(ii + a.Ng) * rowstride
-                          + (long long)s * a.Np;
-    const T* fs = static_cast<const T*>(a.fs);
-    const int n1 = a.Np1, n2 = a.Np2, n3 = a.Np3;
-    for (int c = tid; c < a.Np; c += PTHREADS) fb[c] = fs[cbase + c];
-    for (int q = tid; q < n1 + n2 + n3; q += PTHREADS) {
-        if (q < n1) vg[q] = a.sg.p1_start[s] + (0.5 + q) * a.sg.dp1[s];
-        else if (q < n1 + n2) vg[q] = a.sg.p2_start[s] + (0.5 + (q - n1)) * a.sg.dp2[s];
-        else vg[q] = a.sg.p3_start[s] + (0.5 + (q - n1 - n2)) * a.sg.dp3[s];
-    }
-    const long long plane_g = (long long)a.Nq2g * a.Nq1g;
-    const long long qg = (long long)(jj + a.Ng) * a.Nq1g + (ii + a.Ng);
-    const double E1 = a.cell[0 * plane_g + qg], E2 = a.cell[1 * plane_g + qg];
-    const double E3 = a.cell[2 * plane_g + qg], B1 = a.cell[3 * plane_g + qg];
-    const double B2 = a.cell[4 * plane_g + qg], B3 = a.cell[5 * plane_g + qg];
-    const double em = a.sg.charge[s] / a.sg.mass[s];
-    Weno5Side<T> Sr, Sl;
-    Sr.set(true);
-    Sl.set(false);
-    PDiv D1, D2;
-    D1.set(n1);
-    D2.set(n2);
-    __syncthreads();
-
-    // element c -> (i1, i2, i3)
-    auto split = [&](int c, int& i1, int& i2, int& i3) {
-        const int r12 = D1.div(c, &i1);
-        i3 = D2.div(r12, &i2);
-    };
-    // left-face fluxes of every element along each p axis with more than one
-    // cell (a single-cell axis contributes exactly zero), one pass
-    for (int c = tid; c < a.Np; c += PTHREADS) {
-        int i1, i2, i3;
-        split(c, i1, i2, i3);
-        const double v1 = vg[i1], v2 = vg[n1 + i2], v3 = vg[n1 + n2 + i3];
-        if (n1 > 1)
-            Fx[0][c] = p_face_flux<RECON, EXACT>(fb, c, 1, n1, i1,
-                                                 T(em * ((E1 + v2 * B3) - v3 * B2)), Sr, Sl);
-        if (n2 > 1)
-            Fx[1][c] = p_face_flux<RECON, EXACT>(fb, c, n1, n2, i2,
-                                                 T(em * ((E2 + v3 * B1) - v1 * B3)), Sr, Sl);
-        if (n3 > 1)
-            Fx[2][c] = p_face_flux<RECON, EXACT>(fb, c, n1 * n2, n3, i3,
-                                                 T(em * ((E3 + v1 * B2) - v2 * B1)), Sr, Sl);
-    }
-    __syncthreads();
-    // final combine
-    T* out1 = static_cast<T*>(a.out1);
-    T* out2 = static_cast<T*>(a.out2);
-    const T* base1 = static_cast<const T*>(a.base1);
-    const T* base2 = static_cast<const T*>(a.base2);
-    const T* kq = static_cast<const T*>(a.kq);
-    double macc[kNumMom] = {0, 0, 0, 0, 0};
-    const T c1 = T(a.c1), c2 = T(a.c2);
-    const bool ghost_cell = (a.periodic1 && (ii < a.Ng || ii >= a.Nq1 - a.Ng)) ||
-                            (a.periodic2 && (jj < a.Ng || jj >= a.Nq2 - a.Ng));
-    const T inv1 = T(1.0 / a.sg.dp1[s]), inv2 = T(1.0 / a.sg.dp2[s]);
-    const T inv3 = T(1.0 / a.sg.dp3[s]);
-    for (int c = tid; c < a.Np; c += PTHREADS) {
-        int i1, i2, i3;
-        split(c, i1, i2, i3);
-        // d_a = (F_a(right face) - F_a(left face)) / dp_a, circular along the axis
-        T t1 = T(0), t2 = T(0), t3 = T(0);
-        if (n1 > 1) {
-            const int cn = i1 + 1 < n1 ? c + 1 : c - (n1 - 1);
-            t1 = (Fx[0][cn] - Fx[0][c]) * inv1;
-        }
-        if (n2 > 1) {
-            const int cn = i2 + 1 < n2 ? c + n1 : c - (n2 - 1) * n1;
-            t2 = (Fx[1][cn] - Fx[1][c]) * inv2;
-        }
-        if (n3 > 1) {
-            const int cn = i3 + 1 < n3 ? c + n1 * n2 : c - (n3 - 1) * n1 * n2;
-            t3 = (Fx[2][cn] - Fx[2][c]) * inv3;
-        }
-        const long long g = cbase + c;
-        if (a.term) {
-            // one p-flux divergence (df_dt_fvm.py:325-335 term_to_return)
-            out1[g] = a.term == 1 ? t1 : (a.term == 2 ? t2 : t3);
-            continue;
-        }
-        T kk = kq[g] + (-((t1 + t2) + t3));
-        T o1 = base1 ? base1[g] + kk * c1 : kk;
-        out1[g] = o1;
-        if (out2) out2[g] = base2[g] + kk * c2;
-        if (ghost_cell)
-            write_ghost_images(out1, o1, ii, jj, s, c, a.Ng, a.Nq1, a.Nq2, a.Nq1g, a.Nq2g,
-                               a.periodic1, a.periodic2, rowstride, colstride, a.Np);
-        if (a.flag && !isfinite(double(o1))) atomicOr(a.flag, 1);
-        if (a.mom_out) {
-            const double w1 = vg[i1], w2 = vg[n1 + i2], w3 = vg[n1 + n2 + i3];
-            const double vsq = (w1 * w1 + w2 * w2) + w3 * w3;
-            const double ov = double(o1);
-            macc[0] += ov; macc[1] += ov * w1; macc[2] += ov * w2; macc[3] += ov * w3;
-            macc[4] += (0.5 * ov) * vsq;
-        }
-    }
-    if (a.mom_out) {
-        const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-        for (int q = 0; q < kNumMom; ++q) {
-            double v = warp_sum(macc[q]);
-            if (lane == 0) red[warp][q] = v;
-        }
-        __syncthreads();
-        if (tid < kNumMom) {
-            double v = 0.0;
-            for (int w = 0; w < PTHREADS / 32; ++w) v += red[w][tid];
-            const long long plane = (long long)a.Nq2 * a.Nq1;
-            a.mom_out[((long long)tid * a.Ns + s) * plane + (long long)jj * a.Nq1 + ii] = v;
         }
     }
 }

@@ -4,6 +4,7 @@
 
 #include "launch.h"
 #include "fvm_kernels.cuh"
+#include "pstage_kernel.cuh"
 #include "asl_kernels.cuh"
 
 namespace bolt {
@@ -46,22 +47,23 @@ cudaError_t BOLT_CAT(launch_qstage_, BOLT_SUFFIX)(const QStageArgs& a, int recon
 }
 
 template <int RECON>
-static cudaError_t plaunch(const PStageArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
+static cudaError_t plaunch(const PStageArgs& a, dim3 grid, int threads, size_t smem,
+                           cudaStream_t st) {
     auto k = pstage_kernel<BOLT_T, BOLT_EXACT, RECON>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<grid, PTHREADS, smem, st>>>(a);
+    k<<<grid, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t BOLT_CAT(launch_pstage_, BOLT_SUFFIX)(const PStageArgs& a, int recon, dim3 grid,
-                                                  size_t smem, cudaStream_t st) {
+                                                  int threads, size_t smem, cudaStream_t st) {
     switch (recon) {
-        case BOLT_RECON_PC: return plaunch<BOLT_RECON_PC>(a, grid, smem, st);
-        case BOLT_RECON_MINMOD: return plaunch<BOLT_RECON_MINMOD>(a, grid, smem, st);
-        case BOLT_RECON_PPM: return plaunch<BOLT_RECON_PPM>(a, grid, smem, st);
-        default: return plaunch<BOLT_RECON_WENO5>(a, grid, smem, st);
+        case BOLT_RECON_PC: return plaunch<BOLT_RECON_PC>(a, grid, threads, smem, st);
+        case BOLT_RECON_MINMOD: return plaunch<BOLT_RECON_MINMOD>(a, grid, threads, smem, st);
+        case BOLT_RECON_PPM: return plaunch<BOLT_RECON_PPM>(a, grid, threads, smem, st);
+        default: return plaunch<BOLT_RECON_WENO5>(a, grid, threads, smem, st);
     }
 }
 

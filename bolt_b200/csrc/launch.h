@@ -70,16 +70,71 @@ inline int current_sm_count() {
     return sms;
 }
 
-// the f, flux and two divergence arrays, then the p-cell centres (doubles)
-inline size_t pstage_smem(int Np, size_t elem, int ntab) {
-    return ((4 * (size_t)Np * elem + 7) & ~(size_t)7) + (size_t)ntab * sizeof(double);
+// p-blocks the p-stage takes: four blocks of values and the p-cell centres
+// within 200 KB (6,250 FP64 or 12,600 FP32 p-cells)
+inline bool pstage_fits(int Np, size_t elem, int ntab) {
+    return ((4 * (size_t)Np * elem + 7) & ~(size_t)7) + (size_t)ntab * sizeof(double) <=
+           200 * 1024;
+}
+
+// Launch shape of the p-stage kernel: threads per CTA (one q-cell) and the
+// pieces each p-line is walked in.
+struct PShape {
+    int threads, seg[3];
+    size_t smem;
+};
+
+// A thread's work on one axis is rounds x (piece + 3): a piece costs its cells
+// and about three more for the walker's start.  The shape minimises thread-time
+// of a CTA, scaled up while the SM holds fewer than 24 warps of this launch
+// (latency not hidden): 2D blocks take the fewest threads that still fill the
+// SM, small q-grids take as many threads as shorten the walk.
+inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, long long ctas, int sms) {
+    const int n[3] = {n1, n2, n3};
+    const int Np = n1 * n2 * n3;
+    PShape best;
+    best.smem = 2 * (size_t)pstage_pitch(n1) * n2 * n3 * elem + (size_t)(n1 + n2 + n3) * 8;
+    best.threads = 32;
+    double best_cost = 1e300;
+    const long long by_smem = 233472LL / (long long)(best.smem + 1024 + 640);
+    for (int t = 32; t <= PTHREADS_MAX; t += 32) {
+        if (t > 32 && t > Np) break;
+        long long resident = by_smem < 1 ? 1 : by_smem;
+        if (resident > 2048 / t) resident = 2048 / t;
+        if (resident > 32) resident = 32;
+        const long long have = (ctas + sms - 1) / sms;
+        if (resident > have) resident = have;
+        double cost = 1.5 * ((Np + t - 1) / t);
+        int seg[3] = {1, 1, 1};
+        for (int ax = 0; ax < 3; ++ax) {
+            if (n[ax] == 1) continue;
+            double c_best = 1e300;
+            for (int s = 1; s <= n[ax]; ++s) {
+                const int len = (n[ax] + s - 1) / s;
+                const double c = (double)(((long long)Np / n[ax] * s + t - 1) / t) * (len + 3.0);
+                if (c < c_best - 1e-9) {
+                    c_best = c;
+                    seg[ax] = s;
+                }
+            }
+            cost += c_best;
+        }
+        const double warps = (double)resident * t / 32.0;
+        const double total = cost * t * (warps < 24.0 ? 24.0 / warps : 1.0);
+        if (total < best_cost - 1e-9) {
+            best_cost = total;
+            best.threads = t;
+            for (int ax = 0; ax < 3; ++ax) best.seg[ax] = seg[ax];
+        }
+    }
+    return best;
 }
 
 #define BOLT_DECLARE_LAUNCHERS(SUFFIX, T)                                                   \
     cudaError_t launch_qstage_##SUFFIX(const QStageArgs& a, int recon, int tiling, int bgk, \
                                        dim3 grid, size_t smem, cudaStream_t st);            \
     cudaError_t launch_pstage_##SUFFIX(const PStageArgs& a, int recon, dim3 grid,           \
-                                       size_t smem, cudaStream_t st);                       \
+                                       int threads, size_t smem, cudaStream_t st);          \
     cudaError_t launch_moment_##SUFFIX(const void* f, int mid, double* out, int Ns,          \
                                        int Np1, int Np2, int Np3, int Nq1g, int Nq2g,        \
                                        const SpeciesGrid& sg, cudaStream_t st);             \
