@@ -4,7 +4,7 @@
 
 The FP64 kernels are compiled with -fmad=false so that their arithmetic
 follows the reference's operation order; the FP32 kernels and the FP64
-kernel of the fast FP64 form use FMA and approximate division (FP32) or
+kernel of the fast FP64 form (kernels_f64pair) use FMA and approximate division (FP32) or
 Newton-refined reciprocals (FP64).  The library links the CUDA runtime statically and
 loads cuTensorMapEncodeTiled through the runtime's driver entry point.
 """
@@ -25,6 +25,9 @@ UNITS = [
     ('kernels_f64.cu', ['-fmad=false']),
     ('kernels_f32.cu', ['-prec-div=false', '-prec-sqrt=false', '-ftz=true']),
     ('kernels_f64pair.cu', []),
+    ('kernels_f64exact.cu', ['-fmad=false']),
+    ('kernels_f32any.cu', ['-prec-div=false', '-prec-sqrt=false', '-ftz=true']),
+    ('kernels_f64exactany.cu', ['-fmad=false']),
     ('bolt_capi.cu', []),
     ('bolt_noalloc.cu', []),
     ('bolt_batch.cu', ['-prec-div=false', '-prec-sqrt=false', '-ftz=true']),

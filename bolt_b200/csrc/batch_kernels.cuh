@@ -184,13 +184,13 @@ batch_stage_kernel(const BatchStageArgs a) {
                 const int r0 = j0 + (right ? 0 : 1);
                 float y0 = Xb[r0][lane], y1 = Xb[r0 + 1][lane], y2 = Xb[r0 + 2][lane];
                 float y3 = Xb[r0 + 3][lane], y4 = Xb[r0 + 4][lane];
-                float Fprev = v * W.first(y0, y1, y2, y3, y4, S);
+                float Fprev = v * W.first(y0, y1, y2, y3, y4, right, S);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int j = j0 + q;             // local cell
                     y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                     y4 = Xb[r0 + 5 + q][lane];
-                    const float Fn = v * W.next(y0, y1, y2, y3, y4, S);
+                    const float Fn = v * W.next(y0, y1, y2, y3, y4, right, S);
                     float k = (Fprev - Fn) * inv_dq;
                     Fprev = Fn;
                     const float fc = Xb[j + kBatchNg][lane];

@@ -123,6 +123,7 @@ struct BoltCtx {
     int pair_enabled;       // paired kernel allowed (BOLT_NO_PAIR unset)
     PShape pshape;          // launch shape of the p-stage kernel
     int pair_shape_ok;      // grid/method meet the paired kernel's shape conditions
+    int any_shape_ok;       // ... or those of its form for any grid
 };
 
 #define CK(x)                                             \
@@ -284,24 +285,34 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
     ctx->ntab = g.N_p1 + g.N_p2 + g.N_p3;
     ctx->bgk_direct = (p.p_dim == 1 ||
                        (size_t)t.tq1 * t.tq2 * ctx->ntab * sizeof(double) > 64 * 1024) ? 1 : 0;
-    // the paired kernel's shape conditions (the per-call ones are checked at
-    // launch): FP32, or FP64 in its throughput form
-    ctx->pair_shape_ok = (ctx->elem == 4 || p.dtype == BOLT_F64_FAST) &&
-                         ctx->tiling == TILING_2D && !(ctx->bgk && ctx->bgk_direct) &&
+    // the tile kernels' shape conditions (the per-call ones are checked at
+    // launch): whole tiles and chunks (pair), or any grid with enough ghost
+    // cells for the stencil and one periodic image per cell (any)
+    ctx->any_shape_ok = ctx->tiling == TILING_2D && !(ctx->bgk && ctx->bgk_direct) &&
+                        g.N_ghost >= HALO && 2 * g.N_ghost <= g.N_q1 &&
+                        2 * g.N_ghost <= g.N_q2 && ctx->fcount < (1ull << 31);
+    ctx->pair_shape_ok = ctx->tiling == TILING_2D && !(ctx->bgk && ctx->bgk_direct) &&
                          g.N_q1 % 8 == 0 && g.N_q2 % 8 == 0 && ctx->Np % PW == 0 &&
                          g.N_p1 % 8 == 0 && 2 * g.N_ghost <= g.N_q1 &&
                          2 * g.N_ghost <= g.N_q2 && ctx->fcount < (1ull << 31);
-    if (ctx->pair_shape_ok) {
-        // its shared memory (exp tables grow with N_p1 + N_p2 + N_p3) must fit a CTA
+    if (ctx->pair_shape_ok || ctx->any_shape_ok) {
+        // their shared memory (exp tables grow with N_p1 + N_p2 + N_p3) must fit a CTA
         int dev = 0, optin = 232448;
         if (cudaGetDevice(&dev) == cudaSuccess)
             cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (qpair_smem(ctx->ntab, ctx->bgk, ctx->elem) > (size_t)optin) ctx->pair_shape_ok = 0;
+        if (qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, 1) > (size_t)optin) ctx->any_shape_ok = 0;
     }
     // p-splits: the grid is (q-tiles, species x splits)
     {
-        const size_t smem_est = ctx->pair_shape_ok
-            ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem)
+        // (with fields no q-stage writes moments, and the currents' partial sums
+        // are cut as the scalar kernel cuts them, or the FP32 / FP64-fast tile
+        // kernel where the grid has whole tiles)
+        const bool tiled = p.fields_enabled
+            ? ctx->pair_shape_ok && p.dtype != BOLT_F64
+            : ctx->pair_shape_ok || ctx->any_shape_ok;
+        const size_t smem_est = tiled
+            ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, !ctx->pair_shape_ok)
             : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk, ctx->bgk_direct, ctx->ntab);
         const int nchunks = (ctx->Np + PW - 1) / PW;
         const long long base_ctas = (long long)ctx->ntiles1 * ctx->ntiles2 * g.N_s;
@@ -765,25 +776,26 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
     a.full_chunks = (ctx->Np % PW) == 0;
     a.sg = ctx->sg;
     dim3 grid(ctx->ntiles1 * ctx->ntiles2, g.N_s * ctx->nsplit);
-    // the paired kernel (FP32, or FP64 throughput form) covers the fused 2-D stage with every
-    // buffer reachable by TMA; everything else (FP64, other reconstructions,
-    // 1-D tilings, write-k mode, currents, tau arrays) runs the scalar kernel
+    // the paired kernel covers the fused 2-D stage with every buffer reachable
+    // by TMA; everything else (1-D tilings, write-k mode, currents, tau arrays,
+    // sizes off its tiles) runs the scalar kernel
     // (so do the write-k stages of field-coupled steps, unless they also
     // accumulate currents; bolt_dfdt without fields keeps the scalar kernel,
     // the one bolt_dfdt_noalloc runs, so the two agree to the bit)
-    bool pair = ctx->pair_shape_ok && ctx->pair_enabled && !want_j && a.use_tma &&
-                (write_k ? ctx->p.fields_enabled != 0 : a.base1 != nullptr) &&
-                ctx->tau_arr == nullptr;
-    if (pair) {
-        const void* ptrs[4] = {a.base1, a.out1, a.base2, a.out2};
-        for (int i = 0; i < 4; ++i)
-            if (ptrs[i] && ((uintptr_t)ptrs[i]) % 16 != 0) pair = false;
-        if ((a.base2 == nullptr) != (a.out2 == nullptr)) pair = false;
+    bool tiles = ctx->pair_enabled &&
+                 (write_k ? ctx->p.fields_enabled != 0 : a.base1 != nullptr) &&
+                 ctx->tau_arr == nullptr;
+    if (tiles) {
+        if ((a.base2 == nullptr) != (a.out2 == nullptr)) tiles = false;
         // stage shapes of the paired kernel: bases = stage input, or out2 is
         // its own base (accumulated in place), or no out2
         const bool bx = a.base1 == a.fs && (!a.base2 || a.base2 == a.fs);
-        if (a.base2 && !bx && a.base2 != a.out2) pair = false;
+        if (a.base2 && !bx && a.base2 != a.out2) tiles = false;
     }
+    bool pair = tiles && ctx->pair_shape_ok && !want_j && a.use_tma;
+    const void* ptrs[4] = {a.base1, a.out1, a.base2, a.out2};
+    for (int i = 0; i < 4; ++i)
+        if (ptrs[i] && ((uintptr_t)ptrs[i]) % 16 != 0) pair = false;
     if (pair) {
         // copy each map out at once: a later lookup may recycle its cache slot
         const CUtensorMap* m;
@@ -798,21 +810,43 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         }
     }
     if (region >= 0) {
-        if (!pair) return BOLT_ERR_UNSUPPORTED;
+        // (the reference-order FP64 form runs its stages whole)
+        if (!pair || ctx->p.dtype == BOLT_F64) return BOLT_ERR_UNSUPPORTED;
         const int n1 = ctx->ntiles1, n2 = ctx->ntiles2;
         const int inner = std::max(0, n1 - 2 * a.ext1) * std::max(0, n2 - 2 * a.ext2);
         const int count = region == 0 ? inner : n1 * n2 - inner;
         if (count == 0) return BOLT_OK;
         grid.x = (unsigned)count;
     }
-    const size_t smem = pair ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem)
-                             : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk, ctx->bgk_direct,
-                                           ctx->ntab);
-    cudaError_t e = ctx->elem == 8
-        ? (pair ? launch_qpair_f64(a, ctx->bgk, ctx->recon_q, grid, smem, st)
-                : launch_qstage_f64(a, ctx->recon_q, ctx->tiling, ctx->bgk, grid, smem, st))
-        : (pair ? launch_qpair_f32(a, ctx->bgk, ctx->recon_q, grid, smem, st)
-                : launch_qstage_f32(a, ctx->recon_q, ctx->tiling, ctx->bgk, grid, smem, st));
+    // sizes off the tiles, and the stages that accumulate currents: the same
+    // kernel for any grid (its loads by TMA where rows and base are aligned).
+    // FP32 runs with fields and several species keep the scalar kernel there: a
+    // neutral plasma's current is the difference of nearly equal species
+    // currents, at the level of their FP32 rounding, so another rounding of the
+    // faces would be another electric field (FP64 has the same bits either way)
+    const bool any = tiles && !pair && ctx->any_shape_ok &&
+                     !(ctx->elem == 4 && ctx->p.fields_enabled && g.N_s > 1);
+    if (any && a.use_tma && a.base1) {
+        const CUtensorMap* m = (uintptr_t)a.base1 % 16 == 0
+            ? get_tmap(ctx, a.base1, TMAP_TILE) : nullptr;
+        if (m) a.tm_b1 = *m; else a.use_tma = 0;
+    }
+    const size_t smem = pair || any ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, any)
+                                    : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk,
+                                                  ctx->bgk_direct, ctx->ntab);
+    const int bgk = ctx->bgk, recon = ctx->recon_q;
+    cudaError_t e;
+    if (pair)
+        e = ctx->elem == 4 ? launch_qpair_f32(a, bgk, recon, grid, smem, st)
+            : ctx->p.dtype == BOLT_F64_FAST
+                ? launch_qpair_f64(a, bgk, recon, grid, smem, st)
+                : launch_qpair_f64exact(a, bgk, recon, grid, smem, st);
+    else if (any)
+        e = ctx->elem == 4 ? launch_qpair_f32_any(a, bgk, recon, grid, smem, st)
+                           : launch_qpair_f64exact_any(a, bgk, recon, grid, smem, st);
+    else
+        e = ctx->elem == 4 ? launch_qstage_f32(a, recon, ctx->tiling, bgk, grid, smem, st)
+                           : launch_qstage_f64(a, recon, ctx->tiling, bgk, grid, smem, st);
     ctx->launches++;
     if (pair) ctx->pair_launches++;
     CK(e);

@@ -68,14 +68,14 @@ __host__ __device__ inline QLayout qstage_layout(int tq1, int tq2, int q2, int e
 // itself, hence the 1 KB of slack in total).  FP32: 111.8 KB (two CTAs per
 // SM); FP64: 216.7 KB (one).
 struct PLayout {
-    unsigned x, o1, o2, b1, d1, tabs, vgrid, bars, total;
+    unsigned x, o1, o2, b1, d1, tabs, vgrid, vtab, jacc, bars, total;
 };
 
 constexpr unsigned kPairTileElems = 8 * 8 * PW;                        // one 8x8 tile
 constexpr unsigned kPairHaloElems = (8 + 2 * HALO) * (8 + 2 * HALO) * PW;  // 14x14 halo tile
 constexpr unsigned kTabPitch = 33;       // exp-table row: 32 q-cell pairs + 1 pad
 
-__host__ __device__ inline PLayout qpair_layout(int ntab, int bgk, unsigned elem) {
+__host__ __device__ inline PLayout qpair_layout(int ntab, int bgk, unsigned elem, int any) {
     PLayout L;
     unsigned o = 0;
     const unsigned tile = kPairTileElems * elem;
@@ -88,6 +88,8 @@ __host__ __device__ inline PLayout qpair_layout(int ntab, int bgk, unsigned elem
                                                   // parameters of the 64 q-cells)
     L.tabs = o; o += bgk ? kTabPitch * ntab * 2 * elem : 0u;  // exp tables, a pair per q-cell pair
     L.vgrid = o; o += ntab * sizeof(double);
+    L.vtab = o; o += any ? 2 * 4 * PW * sizeof(double) : 0u;   // chunk velocities
+    L.jacc = o; o += any ? 8 * 8 * 3 * sizeof(double) : 0u;    // currents
     L.bars = qalign(o, 8); o = L.bars + 4 * sizeof(unsigned long long);
     L.total = o + 1024;
     return L;

@@ -55,26 +55,45 @@ template <> struct Consts<float> {
 // is positive, the left-face set otherwise (weno5.py:74-92).
 template <typename T>
 struct Weno5Side {
-    T num1, den1, num2, den2, num3, den3;      // w_k = num_k / ((den_k*beta_k)*beta_k)
-    T cw1, cw2, cw3;                           // num_k / den_k (fast path)
+    T cw1, cw2, cw3;                           // weights' numerators
     T a10, a11, a12, a20, a21, a22, a30, a31, a32;  // u_k = (a_k0 y + a_k1 y) + a_k2 y
     __device__ __forceinline__ void set(bool right) {
         cw2 = T(0.625);
         cw1 = right ? T(0.0625) : T(0.3125);
         cw3 = right ? T(0.3125) : T(0.0625);
         if (right) {
-            num1 = T(1); den1 = T(16); num2 = T(5); den2 = T(8); num3 = T(5); den3 = T(16);
             a10 = T(0.375);  a11 = T(-1.25); a12 = T(1.875);
             a20 = T(-0.125); a21 = T(0.75);  a22 = T(0.375);
             a30 = T(0.375);  a31 = T(0.75);  a32 = T(-0.125);
         } else {
-            num1 = T(5); den1 = T(16); num2 = T(5); den2 = T(8); num3 = T(1); den3 = T(16);
             a10 = T(-0.125); a11 = T(0.75);  a12 = T(0.375);
             a20 = T(0.375);  a21 = T(0.75);  a22 = T(-0.125);
             a30 = T(1.875);  a31 = T(-1.25); a32 = T(0.375);
         }
     }
 };
+
+// 1/x in FP64 for finite normal x: the hardware approximation refined by two
+// Newton-Raphson steps for f(r) = 1/r - x, r <- r + r (1 - x r); each step
+// doubles the number of correct bits, so the last one rounds a value within
+// about 2^-80 of 1/x
+__device__ __forceinline__ double rcp_nr(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    double e = fma(-x, r, 1.0);
+    r = fma(r, e, r);
+    e = fma(-x, r, 1.0);
+    return fma(r, e, r);
+}
+
+// a/b rounded to nearest from r = 1/b rounded to nearest: the quotient a r
+// corrected by its remainder, exact with FMA (Markstein, IBM J. Res. Dev. 34,
+// 1990).  The reference's divisions by the grid spacing and the collision time
+// share their reciprocal this way, and the WENO weights theirs.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-b, q, a), r, q);
+}
 
 // ---------------------------------------------------------------------------
 // WENO5, exact reference order (weno5.py:58-96)
@@ -86,42 +105,12 @@ __device__ __forceinline__ double weno_beta_exact(double a, double b, double c) 
     return poly + 1e-17 * (((1.0 + fabs(a)) + fabs(b)) + fabs(c));
 }
 
-__device__ __forceinline__ double weno5_exact(double y0, double y1, double y2, double y3,
-                                              double y4, const Weno5Side<double>& S) {
-    double b1 = weno_beta_exact(y0, y1, y2);
-    double b2 = weno_beta_exact(y1, y2, y3);
-    double b3 = weno_beta_exact(y2, y3, y4);
-    double w1 = S.num1 / ((S.den1 * b1) * b1);
-    double w2 = S.num2 / ((S.den2 * b2) * b2);
-    double w3 = S.num3 / ((S.den3 * b3) * b3);
-    double den = (w1 + w2) + w3;
-    double u1 = (S.a10 * y0 + S.a11 * y1) + S.a12 * y2;
-    double u2 = (S.a20 * y1 + S.a21 * y2) + S.a22 * y3;
-    double u3 = (S.a30 * y2 + S.a31 * y3) + S.a32 * y4;
-    return ((w1 * u1 + w2 * u2) + w3 * u3) / den;
-}
-
 // WENO5, fast FP32 form
 __device__ __forceinline__ float weno_beta_fast(float a, float b, float c) {
     float d1 = fmaf(-2.0f, b, a + c);           // a - 2b + c
     float d2 = fmaf(3.0f, c, fmaf(-4.0f, b, a));  // a - 4b + 3c
     float e = fmaf(1e-17f, fabsf(a) + fabsf(b) + fabsf(c), 1e-17f);
     return fmaf(13.0f / 12.0f * d1, d1, fmaf(0.25f * d2, d2, e));
-}
-
-__device__ __forceinline__ float weno5_fast(float y0, float y1, float y2, float y3, float y4,
-                                            const Weno5Side<float>& S) {
-    float r1 = fast_rcp(weno_beta_fast(y0, y1, y2));
-    float r2 = fast_rcp(weno_beta_fast(y1, y2, y3));
-    float r3 = fast_rcp(weno_beta_fast(y2, y3, y4));
-    float w1 = S.cw1 * r1 * r1;
-    float w2 = S.cw2 * r2 * r2;
-    float w3 = S.cw3 * r3 * r3;
-    float u1 = fmaf(S.a12, y2, fmaf(S.a11, y1, S.a10 * y0));
-    float u2 = fmaf(S.a22, y3, fmaf(S.a21, y2, S.a20 * y1));
-    float u3 = fmaf(S.a32, y4, fmaf(S.a31, y3, S.a30 * y2));
-    float num = fmaf(w3, u3, fmaf(w2, u2, w1 * u1));
-    return num * fast_rcp(w1 + w2 + w3);
 }
 
 // ---------------------------------------------------------------------------
@@ -171,25 +160,19 @@ __device__ __forceinline__ T ppm_face(T y0, T y1, T y2, T y3, T y4, bool right) 
 }
 
 // ---------------------------------------------------------------------------
-// Unified face value of cell y2 (right face if `right`, else left face)
+// Face value of cell y2 (right face if `right`, else left face) of the
+// reconstructions that carry no state
 // ---------------------------------------------------------------------------
-template <int RECON, bool EXACT, typename T>
-__device__ __forceinline__ T face_value(T y0, T y1, T y2, T y3, T y4, bool right,
-                                        const Weno5Side<T>& S) {
+template <int RECON, typename T>
+__device__ __forceinline__ T face_value(T y0, T y1, T y2, T y3, T y4, bool right) {
+    static_assert(RECON != BOLT_RECON_WENO5, "WENO5 faces: Weno5Walker");
     if (RECON == BOLT_RECON_PC) {
         return y2;
     } else if (RECON == BOLT_RECON_MINMOD) {
         T s = minmod_slope(y1, y2, y3);
         return right ? y2 + T(0.5) * s : y2 - T(0.5) * s;
-    } else if (RECON == BOLT_RECON_PPM) {
-        return ppm_face(y0, y1, y2, y3, y4, right);
     } else {
-        if constexpr (EXACT) {
-            return weno5_exact(double(y0), double(y1), double(y2), double(y3), double(y4),
-                               reinterpret_cast<const Weno5Side<double>&>(S));
-        } else {
-            return weno5_fast(y0, y1, y2, y3, y4, S);
-        }
+        return ppm_face(y0, y1, y2, y3, y4, right);
     }
 }
 
@@ -197,38 +180,54 @@ __device__ __forceinline__ T face_value(T y0, T y1, T y2, T y3, T y4, bool right
 // WENO5 along a sliding window.  Consecutive faces share two of their three
 // substencils: beta_1 of face f+1 is beta_2 of face f and beta_2 of face f+1
 // is beta_3 of face f, so each step computes one new smoothness indicator.
-// The exact flavour reuses the identical FP64 values (bit-for-bit the same
-// as recomputing them); the fast flavour carries 1/beta^2.
+// The fast flavour carries 1/beta^2.
 // ---------------------------------------------------------------------------
 template <bool EXACT, typename T> struct Weno5Walker;
 
+// The exact flavour carries, per substencil, the two quotients that the
+// reference's weights num / ((den beta) beta) are made of: with B = beta beta,
+// num in {1, 5} and den a power of two, w = (1/B or 5/B) * 2^-n bit for bit
+// (scaling by a power of two is exact), and the common factor 16 of the three
+// weights cancels exactly in the normalised sum.  So a face costs one
+// reciprocal for its new substencil and one for the sum, instead of four
+// divisions, and its value has the bits of the reference's expressions.  B is
+// capped where its reciprocal would leave the normal range.
 template <> struct Weno5Walker<true, double> {
-    double b2, b3;
-    __device__ __forceinline__ double eval(double b1, double y0, double y1, double y2, double y3,
-                                           double y4, const Weno5Side<double>& S) {
-        double w1 = S.num1 / ((S.den1 * b1) * b1);
-        double w2 = S.num2 / ((S.den2 * b2) * b2);
-        double w3 = S.num3 / ((S.den3 * b3) * b3);
-        double den = (w1 + w2) + w3;
-        double u1 = (S.a10 * y0 + S.a11 * y1) + S.a12 * y2;
-        double u2 = (S.a20 * y1 + S.a21 * y2) + S.a22 * y3;
-        double u3 = (S.a30 * y2 + S.a31 * y3) + S.a32 * y4;
-        return ((w1 * u1 + w2 * u2) + w3 * u3) / den;
+    double r2, t2, r3, t3;                     // 1/B and 5/B of substencils 2 and 3
+    __device__ __forceinline__ static void quotients(double beta, double& r, double& t) {
+        const double B = fmin(beta * beta, 1e300);
+        r = rcp_nr(B);
+        t = div_by(5.0, B, r);
+    }
+    __device__ __forceinline__ double eval(double r1, double t1, double y0, double y1, double y2,
+                                           double y3, double y4, bool right,
+                                           const Weno5Side<double>& S) const {
+        // 16 w_k: right faces 1, 10, 5 over B, left faces 5, 10, 1
+        const double w1 = right ? r1 : t1;
+        const double w2 = t2 + t2;
+        const double w3 = right ? t3 : r3;
+        const double den = (w1 + w2) + w3;
+        const double u1 = (S.a10 * y0 + S.a11 * y1) + S.a12 * y2;
+        const double u2 = (S.a20 * y1 + S.a21 * y2) + S.a22 * y3;
+        const double u3 = (S.a30 * y2 + S.a31 * y3) + S.a32 * y4;
+        return div_by((w1 * u1 + w2 * u2) + w3 * u3, den, rcp_nr(den));
     }
     __device__ __forceinline__ double first(double y0, double y1, double y2, double y3, double y4,
-                                            const Weno5Side<double>& S) {
-        double b1 = weno_beta_exact(y0, y1, y2);
-        b2 = weno_beta_exact(y1, y2, y3);
-        b3 = weno_beta_exact(y2, y3, y4);
-        return eval(b1, y0, y1, y2, y3, y4, S);
+                                            bool right, const Weno5Side<double>& S) {
+        double r1, t1;
+        quotients(weno_beta_exact(y0, y1, y2), r1, t1);
+        quotients(weno_beta_exact(y1, y2, y3), r2, t2);
+        quotients(weno_beta_exact(y2, y3, y4), r3, t3);
+        return eval(r1, t1, y0, y1, y2, y3, y4, right, S);
     }
     // window shifted by one cell: y0..y3 are the previous y1..y4
     __device__ __forceinline__ double next(double y0, double y1, double y2, double y3, double y4,
-                                           const Weno5Side<double>& S) {
-        double b1 = b2;
-        b2 = b3;
-        b3 = weno_beta_exact(y2, y3, y4);
-        return eval(b1, y0, y1, y2, y3, y4, S);
+                                           bool right, const Weno5Side<double>& S) {
+        const double r1 = r2, t1 = t2;
+        r2 = r3;
+        t2 = t3;
+        quotients(weno_beta_exact(y2, y3, y4), r3, t3);
+        return eval(r1, t1, y0, y1, y2, y3, y4, right, S);
     }
 };
 
@@ -247,14 +246,14 @@ template <> struct Weno5Walker<false, float> {
         float num = fmaf(w3, u3, fmaf(w2, u2, w1 * u1));
         return num * fast_rcp(w1 + w2 + w3);
     }
-    __device__ __forceinline__ float first(float y0, float y1, float y2, float y3, float y4,
+    __device__ __forceinline__ float first(float y0, float y1, float y2, float y3, float y4, bool,
                                            const Weno5Side<float>& S) {
         float q1 = inv_sq(weno_beta_fast(y0, y1, y2));
         q2 = inv_sq(weno_beta_fast(y1, y2, y3));
         q3 = inv_sq(weno_beta_fast(y2, y3, y4));
         return eval(q1, y0, y1, y2, y3, y4, S);
     }
-    __device__ __forceinline__ float next(float y0, float y1, float y2, float y3, float y4,
+    __device__ __forceinline__ float next(float y0, float y1, float y2, float y3, float y4, bool,
                                           const Weno5Side<float>& S) {
         float q1 = q2;
         q2 = q3;
@@ -270,13 +269,13 @@ struct FaceWalker {
     Weno5Walker<EXACT, T> w;
     __device__ __forceinline__ T first(T y0, T y1, T y2, T y3, T y4, bool right,
                                        const Weno5Side<T>& S) {
-        if (RECON == BOLT_RECON_WENO5) return w.first(y0, y1, y2, y3, y4, S);
-        return face_value<RECON, EXACT>(y0, y1, y2, y3, y4, right, S);
+        if constexpr (RECON == BOLT_RECON_WENO5) return w.first(y0, y1, y2, y3, y4, right, S);
+        else return face_value<RECON>(y0, y1, y2, y3, y4, right);
     }
     __device__ __forceinline__ T next(T y0, T y1, T y2, T y3, T y4, bool right,
                                       const Weno5Side<T>& S) {
-        if (RECON == BOLT_RECON_WENO5) return w.next(y0, y1, y2, y3, y4, S);
-        return face_value<RECON, EXACT>(y0, y1, y2, y3, y4, right, S);
+        if constexpr (RECON == BOLT_RECON_WENO5) return w.next(y0, y1, y2, y3, y4, right, S);
+        else return face_value<RECON>(y0, y1, y2, y3, y4, right);
     }
 };
 
@@ -297,18 +296,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f), a); }
 __device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(fast_rcp(a.x), fast_rcp(a.y)); }
-
-// 1/x in FP64 for finite normal x: the hardware approximation refined by two
-// Newton-Raphson steps for f(r) = 1/r - x, r <- r + r (1 - x r); each step
-// doubles the number of correct bits, the last one lands within an ulp
-__device__ __forceinline__ double rcp_nr(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-x, r, 1.0);
-    return fma(r, e, r);
-}
 
 __device__ __forceinline__ double2 f2(double a) { return make_double2(a, a); }
 __device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
@@ -556,6 +543,22 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) 
                    "l"(gmem_src) : "memory");
 }
 
+__device__ __forceinline__ void cp_async_elem(float* smem_dst, const float* gmem_src) {
+    cp_async4(smem_dst, gmem_src);
+}
+__device__ __forceinline__ void cp_async_elem(double* smem_dst, const double* gmem_src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+                 ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
+                   "l"(gmem_src) : "memory");
+}
+
+// this thread's copies so far arrive on the mbarrier once they have landed (one
+// arrival of the count the barrier was initialised with)
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];"
+                 ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(bar))) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_commit() {
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -563,6 +566,11 @@ __device__ __forceinline__ void cp_async_commit() {
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// all of this thread's copies, in groups or not
+__device__ __forceinline__ void cp_async_wait_everything() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------

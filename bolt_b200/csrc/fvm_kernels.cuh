@@ -297,6 +297,8 @@ qstage_kernel(const __grid_constant__ QStageArgs a) {
     const T* base2 = static_cast<const T*>(a.base2);
     const T* tau_arr = static_cast<const T*>(a.tau_arr);
     const T c1 = T(a.c1), c2 = T(a.c2);
+    // (an infinite collision time: 0 and 0, which divide to 0)
+    const double tau = isinf(a.tau) ? 0.0 : a.tau;
     const T inv_tau = T(1.0 / a.tau);
     const T inv_dq1 = T(1.0 / a.dq1), inv_dq2 = T(1.0 / a.dq2);
     const double mneg = -a.sg.mass[s];
@@ -387,7 +389,7 @@ qstage_kernel(const __grid_constant__ QStageArgs a) {
                     T fn = W.next(y0, y1, y2, y3, y4, right, S);
                     T Fn = v1 * fn;
                     T d;
-                    if (EXACT) d = (-(Fn - Fprev)) / T(a.dq1);
+                    if constexpr (EXACT) d = div_by(-(Fn - Fprev), a.dq1, inv_dq1);
                     else d = (Fprev - Fn) * inv_dq1;
                     stage[(jr * TQ1 + cc) * PWP + lane] = d;
                     if (want_j) {
@@ -446,7 +448,7 @@ qstage_kernel(const __grid_constant__ QStageArgs a) {
                         y4 = colw[(r + 5) * HX * PW];
                         T fn = W.next(y0, y1, y2, y3, y4, right, S);
                         T Fn = v2 * fn;
-                        if (EXACT) kq = kq - (Fn - Fprev) / T(a.dq2);
+                        if constexpr (EXACT) kq = kq - div_by(Fn - Fprev, a.dq2, inv_dq2);
                         else kq = kq - (Fn - Fprev) * inv_dq2;
                         Fprev = Fn;
                         fprev = fn;
@@ -473,8 +475,9 @@ qstage_kernel(const __grid_constant__ QStageArgs a) {
                             fmb = (tb[toff1] * tb[toff2]) * tb[toff3];
                         }
                         if (EXACT) {
-                            double tauv = tau_arr ? double(tau_arr[cvalid ? gidx : 0]) : a.tau;
-                            kk = T(double(kk) + (-(double(fcell) - fmb) / tauv));
+                            const double x = -(double(fcell) - fmb);
+                            kk = T(double(kk) + (tau_arr ? x / double(tau_arr[cvalid ? gidx : 0])
+                                                         : div_by(x, tau, inv_tau)));
                         } else {
                             T itau = tau_arr ? T(1) / tau_arr[cvalid ? gidx : 0] : inv_tau;
                             kk = kk + (T(fmb) - fcell) * itau;

@@ -9,7 +9,7 @@ namespace bolt {
 
 cudaError_t launch_qpair_f64(const QStageArgs& a, int bgk, int recon, dim3 grid, size_t smem,
                              cudaStream_t st) {
-    return launch_qpair<double>(a, bgk, recon, grid, smem, st);
+    return launch_qpair<double, false, QG_TILES>(a, bgk, recon, grid, smem, st);
 }
 
 }  // namespace bolt

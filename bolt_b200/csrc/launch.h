@@ -30,8 +30,9 @@ inline size_t qstage_smem(int tiling, size_t elem, int bgk, int bgk_direct, int 
 }
 
 // bytes of dynamic shared memory of the paired kernel (elem: 4 FP32, 8 FP64)
-inline size_t qpair_smem(int ntab, int bgk, size_t elem) {
-    return qpair_layout(ntab, bgk, (unsigned)elem).total;
+// (any: the form for any grid)
+inline size_t qpair_smem(int ntab, int bgk, size_t elem, int any = 0) {
+    return qpair_layout(ntab, bgk, (unsigned)elem, any).total;
 }
 
 // p-split of the q-stage grid (q-tiles x species x splits): the split that
@@ -182,6 +183,17 @@ cudaError_t launch_qpair_f32(const QStageArgs& a, int bgk, int recon, dim3 grid,
                              cudaStream_t st);
 cudaError_t launch_qpair_f64(const QStageArgs& a, int bgk, int recon, dim3 grid, size_t smem,
                              cudaStream_t st);
+
+// the same FP64 stage in the reference's operation order (BOLT_F64)
+cudaError_t launch_qpair_f64exact(const QStageArgs& a, int bgk, int recon, dim3 grid, size_t smem,
+                                  cudaStream_t st);
+
+// any grid: partial tiles and chunks, and (a.want_j) currents; FP64 in the
+// reference's operation order (both FP64 forms)
+cudaError_t launch_qpair_f32_any(const QStageArgs& a, int bgk, int recon, dim3 grid, size_t smem,
+                                 cudaStream_t st);
+cudaError_t launch_qpair_f64exact_any(const QStageArgs& a, int bgk, int recon, dim3 grid,
+                                      size_t smem, cudaStream_t st);
 
 // FDTD sequence (FP64): prepare -> halo -> E -> halo -> B -> to_cell
 cudaError_t launch_fdtd(const FieldArgs& a, cudaStream_t st, long long* launches);

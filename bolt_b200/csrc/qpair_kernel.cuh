@@ -39,6 +39,27 @@
 // C), at most 128 registers, so that twice the warps hide the FP64 latencies
 // that a single 8-warp CTA left exposed.
 //
+// EXACT (FP64, built without FMA contraction): the arithmetic of the scalar stage
+// kernel, operation by operation, so that a value has the same bits whichever
+// kernel writes it: the reference's operation order and divisions (div_by), table
+// entries by their own exp, and the source term added after both flux
+// differences as the reference does: the q1 walkers put it beside the D1 tile in
+// the out2 staging tile, and a second output that is stored (first RK4 stage)
+// goes from the q2 walkers' registers to memory.  The scalar kernel (8 warps,
+// four divisions a face, single-buffered halo) left the FP64 pipe idle most of
+// the time: an RK4 step of 64^2 x 24^3 cells took 9.62 ms, here 3.78 ms (its
+// bytes alone 1.2 ms); what bounds it now is the latency of the dependent FP64
+// chains at 16 warps per SM.
+//
+// QG_ANY, QG_CURRENTS: any grid.  The halo and base tiles come by TMA where rows
+// are multiples of 16 bytes (cells outside the array read as zero), else by
+// asynchronous copies of single values that arrive on the same barriers; the
+// outputs go from the q2 walkers' registers to memory under a mask, and the
+// accumulator's increment by one red.global.add per element.  An RK2 step of
+// 75 x 50 x 45 x 35 FP32 cells between mirrors (rows of 6300 bytes, by copies)
+// took 551 us on the scalar kernel, here 186 us; a currents stage of 64^2 x 32^2
+// FP32 cells went from 78 to about 35 us.
+//
 // Launch conditions (checked by the host): FP32 or FP64, any reconstruction in q, 8x8 tiling,
 // N_q1, N_q2 multiples of 8 and at least 2 N_g, N_p multiple of 32, N_p1
 // multiple of 8, BGK by exp tables, all five buffers 16-byte aligned, f with
@@ -97,7 +118,8 @@ __device__ __forceinline__ double2 mk2(double a, double b) { return make_double2
 // pairs over q-cell pairs P = m*8 + col (cells of rows 2m and 2m+1 in one tile
 // column, the pair a q1 walker holds): tab[q*kTabPitch + P], the pitch of 33
 // pairs keeping a warp's reads of different q (one per lane) on distinct banks.
-template <typename E, bool BGK, int NT>
+// EXACT: every table entry by its own exp in the reference's expressions.
+template <typename E, bool BGK, int NT, bool EXACT, bool GEN>
 __device__ __forceinline__ void qpair_prologue(const QStageArgs& a, int s, int i0, int j0,
                                                double* vgrid, double* qc,
                                                typename PairOf<E>::P* tabs, int p3lo, int n3) {
@@ -126,7 +148,8 @@ __device__ __forceinline__ void qpair_prologue(const QStageArgs& a, int s, int i
                                 (long long)jj * a.Nq1 + ii;
             const double* src4 = src + 4 * (long long)a.Ns * plane;
             double v = 0.0, v4 = 0.0;
-            const int n = a.nsplit_in;
+            // (cells of a partial tile outside the grid: zero moments)
+            const int n = !GEN || (ii < a.Nq1 && jj < a.Nq2) ? a.nsplit_in : 0;
             int sp = 0;
             if (q == 0) {
                 for (; sp + 4 <= n; sp += 4) {
@@ -158,10 +181,21 @@ __device__ __forceinline__ void qpair_prologue(const QStageArgs& a, int s, int i
         }
         __syncthreads();
         for (int c = tid; c < 64; c += NT)
-            bgk_params_from_sums<true>(a, s, mm + c * kNumMom, qc + c * 5);
+            bgk_params_from_sums<!EXACT>(a, s, mm + c * kNumMom, qc + c * 5);
     }
     __syncthreads();
-    if (BGK) {
+    if (BGK && EXACT) {
+        const double m = a.sg.mass[s];
+        const int n12 = Np1 + Np2;
+        E* tel = reinterpret_cast<E*>(tabs);
+        for (int t = tid; t < 64 * (n12 + n3); t += NT) {
+            const int c = t & 63, r = t >> 6;
+            E* col = tel + 2 * ((c >> 4) * 8 + (c & 7)) + ((c >> 3) & 1);
+            col[2 * kTabPitch * r] =
+                E(bgk_table_entry(a, qc + c * 5, vgrid, r < n12 ? r : r + p3lo, m));
+        }
+    }
+    if (BGK && !EXACT) {
         // One (q-cell, axis) per thread: the axis's exp factors
         // e_j = exp(-beta x_j^2), x_j = v_j - u, beta = m / (2 kB T), from the
         // row nearest u outwards by e_{j+1} = e_j g_j, g_{j+1} = g_j exp(-2 beta dv^2)
@@ -272,9 +306,15 @@ __device__ __forceinline__ void qpair_tile(const QStageArgs& a, int bx, int& t1,
 //           a TMA reduce-add (no base2 load)
 //   QP_K    out1 = k itself (the q-part of df/dt when a p-stage follows: fields
 //           enabled), no base, no moments
+// What the grid looks like:
+//   QG_TILES    whole 8x8 tiles, whole chunks, p1 rows of whole groups of 8
+//   QG_ANY      any size: partial tiles and chunks, any N_p1, any alignment
+//   QG_CURRENTS as QG_ANY, for QP_K, with the partial currents of the stage input
+enum QPairGrid { QG_TILES = 0, QG_ANY = 1, QG_CURRENTS = 2 };
+
 enum QPairMode { QP_X1 = 0, QP_X2 = 1, QP_B1 = 2, QP_B1R2 = 3, QP_K = 4 };
 
-template <typename E, bool BGK, int MODE, int RECON, int ROWS>
+template <typename E, bool BGK, int MODE, int RECON, int ROWS, bool EXACT, int GEN>
 __global__ void __launch_bounds__(ROWS == 2 ? NTHREADS : 2 * NTHREADS,
                                   (sizeof(E) == 4 && ROWS == 2) ? 2 : 1)
 qpair_kernel(const __grid_constant__ QStageArgs a) {
@@ -289,12 +329,16 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             typename std::conditional<RECON == BOLT_RECON_PC, ConstPairWalkerT<E, P>,
                                       Weno5PairWalkerT<E, P>>::type>::type>::type;
     typedef Weno5PairT<E, P> Side;
+    typedef FaceWalker<RECON, true, double> ExactWalker;
     typedef typename PairOf<E>::P TabP;               // table entries: row pairs
     constexpr int NT = ROWS == 2 ? NTHREADS : 2 * NTHREADS;
     constexpr int CS = PairStage<E>::CS, VE = PairStage<E>::VE;
     constexpr bool F64 = sizeof(E) == 8;
     constexpr bool BX = MODE == QP_X1 || MODE == QP_X2 || MODE == QP_K;   // no base tiles
     constexpr bool KOUT = MODE == QP_K;
+    constexpr bool ANY = GEN != QG_TILES, JCUR = GEN == QG_CURRENTS;
+    static_assert(!JCUR || KOUT, "currents: the stages whose q-part is written alone");
+    static_assert(!EXACT || F64, "the reference's operation order: FP64");
     constexpr bool HAS2 = MODE == QP_X2 || MODE == QP_B1R2;
     constexpr bool RED2 = MODE == QP_B1R2;
     constexpr int TQ = 8, HX = TQ + 2 * HALO, NQ = TQ * TQ, NWARP = NT / 32;
@@ -306,7 +350,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     const int Np1 = a.Np1, Np2 = a.Np2, Np = a.Np, Ng = a.Ng;
     const int Nq1 = a.Nq1, Nq2 = a.Nq2;
     const int ntab = Np1 + Np2 + a.Np3;
-    const PLayout Lo = qpair_layout(ntab, BGK, sizeof(E));
+    const PLayout Lo = qpair_layout(ntab, BGK, sizeof(E), ANY);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     E* X = reinterpret_cast<E*>(sm + Lo.x);
@@ -324,7 +368,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     const int s = blockIdx.y / a.nsplit, split = blockIdx.y % a.nsplit;
     const int i0 = tile1 * TQ, j0 = tile2 * TQ;
     const int k_begin = split * a.chunks_per_split;
-    const int k_end = min(Np / PW, k_begin + a.chunks_per_split);
+    const int k_end = min(ANY ? (Np + PW - 1) / PW : Np / PW, k_begin + a.chunks_per_split);
     const int xs = s * Np;                           // TMA x coordinate of the species
     const bool peer2 = a.peer_lo != nullptr;          // q2 images go to the neighbours
     const bool peer1 = a.peer_left != nullptr;        // q1 images go to the neighbours
@@ -332,16 +376,21 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                         ((a.periodic2 || peer2) && (j0 < Ng || j0 + TQ > Nq2 - Ng));
 
     if (tid == 0) {
-        prefetch_tmap(&a.tmap);
-        prefetch_tmap(&a.tm_b1);
-        prefetch_tmap(&a.tm_o1);
-        prefetch_tmap(&a.tm_o2);
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        mbar_init(&bars[2], 1);
-        mbar_init(&bars[3], 1);
+        if (!ANY || a.use_tma) {
+            prefetch_tmap(&a.tmap);
+            if (!ANY || !BX) prefetch_tmap(&a.tm_b1);
+        }
+        if (!ANY) {
+            prefetch_tmap(&a.tm_o1);
+            prefetch_tmap(&a.tm_o2);
+        }
+        // one arrival by the TMA issuer, or one per thread that copies
+        const unsigned arrivals = ANY && !a.use_tma ? NT : 1;
+        for (int b = 0; b < 4; ++b) mbar_init(&bars[b], arrivals);
         fence_barrier_init();
     }
+    const bool copies = ANY && !a.use_tma;   // tiles by per-thread copies, not TMA
+    if (copies) __syncthreads();             // every thread arrives on the barriers
 
     bool failed = false;
     unsigned pend = 0u;        // thread 0: barriers with a load in flight
@@ -360,9 +409,35 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             tma_load_3d(b1s + b * TE, &a.tm_b1, &bars[2 + b], xs + k * PW, i0 + Ng, j0 + Ng);
         }
     };
+    // the same tiles by asynchronous copies of single values, for rows that are
+    // not a multiple of 16 bytes; each thread's copies arrive on the barrier as
+    // they land.  Cells outside the array and p beyond the species are read at
+    // the nearest valid one (never used).
+    auto copy_box = [&](E* dst, const void* src, int k, int g1, int g2, int nx, int half,
+                        uint64_t* bar) {
+        // item: half a row of the box (nx / 2 = half cells), one warp each
+        const E* f = static_cast<const E*>(src) + xs + min(k * PW + lane, Np - 1);
+        const long long rs = (long long)a.Ns * Np, cs = rs * a.Nq1g;
+        for (int item = warp; item < 2 * nx; item += NWARP) {
+            const int hy = item >> 1, h0 = (item & 1) * half;
+            const E* row = f + min(g2 + hy, a.Nq2g - 1) * cs;
+            E* d = dst + (hy * nx + h0) * PW + lane;
+            for (int hx = 0; hx < half; ++hx)
+                cp_async_elem(d + hx * PW, row + min(g1 + h0 + hx, a.Nq1g - 1) * rs);
+        }
+        cp_async_arrive(bar);
+    };
+    auto copy_tiles = [&](int k, int b) {
+        if (k >= k_end || a.stall_test) return;
+        copy_box(X + b * XT, a.fs, k, i0 + Ng - HALO, j0 + Ng - HALO, HX, HX / 2, &bars[b]);
+        if (!BX) copy_box(b1s + b * TE, a.base1, k, i0 + Ng, j0 + Ng, TQ, TQ / 2, &bars[2 + b]);
+    };
     // the first tiles load while the tables are built: thread 0 initialised
     // the barriers itself, the other threads reach them after the prologue
-    if (tid == 0) {
+    if (copies) {
+        copy_tiles(k_begin, 0);
+        copy_tiles(k_begin + 1, 1);
+    } else if (tid == 0) {
         load_x(k_begin, 0);
         load_x(k_begin + 1, 1);
         load_b(k_begin, 0);
@@ -370,14 +445,17 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     }
     // p3 rows of this CTA's p-range (the tables hold only those)
     const int p3lo = (k_begin * PW) / (Np1 * Np2);
-    const int n3 = k_begin < k_end ? (k_end * PW - 1) / (Np1 * Np2) - p3lo + 1 : 0;
-    qpair_prologue<E, BGK, NT>(a, s, i0, j0, vgrid, reinterpret_cast<double*>(d1s), tabs, p3lo,
+    const int p_last = ANY ? min(k_end * PW, Np) - 1 : k_end * PW - 1;
+    const int n3 = k_begin < k_end ? p_last / (Np1 * Np2) - p3lo + 1 : 0;
+    qpair_prologue<E, BGK, NT, EXACT, ANY>(a, s, i0, j0, vgrid, reinterpret_cast<double*>(d1s), tabs, p3lo,
                                n3);
 
     E* __restrict__ out1 = static_cast<E*>(a.out1);
     const P c1 = LaneOf<P>::splat(E(a.c1)), c2 = LaneOf<P>::splat(E(a.c2));
     const E inv_dq1 = E(1.0 / a.dq1), inv_dq2 = E(1.0 / a.dq2);
     const P inv_tau = LaneOf<P>::splat(E(1.0 / a.tau));
+    // EXACT: the divisor beside its reciprocal (an infinite collision time: 0 and 0)
+    const double tau = isinf(a.tau) ? 0.0 : a.tau;
     const bool want_mom = a.mom_out != nullptr;
     const bool check = a.flag != nullptr;
     const unsigned rowstride = (unsigned)(a.Ns * Np);
@@ -404,6 +482,19 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     // columns 2(w-4), 2(w-4)+1; single rows: q1 walkers (warps 0-7) row w, q2
     // walkers (warps 8-15) column w-8; each walks the 8 cells of its line
     const bool q1w = warp < NWARP / 2;
+    // currents of the chunks so far, [q-cell][3]: a warp's sum over the 32 p of
+    // each chunk, added chunk by chunk (face value * v1 at left faces and f * v3
+    // by the q1 walkers, face value * v2 at bottom faces by the q2 walkers)
+    double* jacc = reinterpret_cast<double*>(sm + Lo.jacc);
+    if (JCUR)
+        for (int c = tid; c < NQ * 3; c += NT) jacc[c] = 0.0;
+    auto add_current = [&](int cell, int comp, double v) {
+        v = warp_sum(v);
+        if (lane == 0) jacc[cell * 3 + comp] += v;
+    };
+    // any N_p1: velocities of the chunk's 32 p for phase C, by chunk parity
+    double* vtab = reinterpret_cast<double*>(sm + Lo.vtab);
+    const bool vt_on = ANY && !KOUT && Np1 % 8 != 0;
     const bool pc_on = ROWS == 2 || !q1w;             // this warp runs phase C
     const int lp = ROWS == 2 ? 2 * (warp & 3) : (warp & 7);   // first row / column
     const int sw0 = stg<E>(lp, lane) - lp * CS;       // swizzled lane slot, column lp
@@ -454,7 +545,18 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
         if (!failed && !mbar_wait_bounded(&bars[buf], buf ? phx1 : phx0, a.wait_cycles))
             failed = true;
         const E* Xb = X + buf * XT;
+        // (p beyond the last p-cell: the last p3 row's velocities, never stored)
+        const bool pvalid = !ANY || k * PW + lane < Np;
+        const int jp3 = ANY ? min(ip3, a.Np3 - 1) : ip3;
         const double V1 = vgrid[ip1], V2 = vgrid[Np1 + ip2];
+        if (vt_on && warp == 0) {
+            const double V3 = vgrid[Np1 + Np2 + jp3];
+            double* v = vtab + buf * 4 * PW + lane;
+            v[0] = V1;
+            v[PW] = V2;
+            v[2 * PW] = V3;
+            v[3 * PW] = fma(V1, V1, fma(V2, V2, V3 * V3));
+        }
 
         if (q1w) {
             // ---- q1 faces of rows lp, lp+1, BGK -> D1 --------------------------
@@ -469,19 +571,57 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             P y2 = ld(ra + 2 * PW, rb);
             P y3 = ld(ra + 3 * PW, rb);
             P y4 = ld(ra + 4 * PW, rb);
-            Walker W;
-            const P vq = LaneOf<P>::splat(E(0.5) * v1 * inv_dq1);   // walker: 2x face value
-            P Fprev = W.first(y0, y1, y2, y3, y4, S);
             E* da = d1s + lp * TQ * PW + lane;
             const P* t1 = tb_row + ip1 * kTabPitch * TW;
             const P* t2 = tb_row + (Np1 + ip2) * kTabPitch * TW;
-            const P* t3 = tb_row + (Np1 + Np2 + ip3 - p3lo) * kTabPitch * TW;
+            const P* t3 = tb_row + (Np1 + Np2 + jp3 - p3lo) * kTabPitch * TW;
+            const double V3 = JCUR ? vgrid[Np1 + Np2 + jp3] : 0.0;
+            if constexpr (EXACT) {
+                Weno5Side<double> SX;
+                SX.set(right);
+                ExactWalker WX;
+                double fp = WX.first(y0, y1, y2, y3, y4, right, SX);
+                double Fp = v1 * fp;
+                double* db = o2s + lp * TQ * PW + lane;
+#pragma unroll 1
+                for (int c = 0; c < TQ; ++c) {
+                    y0 = y1; y1 = y2; y2 = y3; y3 = y4;
+                    y4 = ra[(c + 5) * PW];
+                    const double fn = WX.next(y0, y1, y2, y3, y4, right, SX);
+                    const double Fn = v1 * fn;
+                    const double fcell = right ? y2 : y1;
+                    da[c * PW] = div_by(-(Fn - Fp), a.dq1, inv_dq1);
+                    if (BGK) {
+                        const double f0 = (t1[c * TW] * t2[c * TW]) * t3[c * TW];
+                        db[c * PW] = div_by(-(fcell - f0), tau, inv_tau);
+                    }
+                    if (JCUR) {
+                        add_current(lp * TQ + c, 0, pvalid ? fp * V1 : 0.0);
+                        add_current(lp * TQ + c, 2, pvalid ? fcell * V3 : 0.0);
+                    }
+                    Fp = Fn;
+                    fp = fn;
+                }
+            } else {
+            Walker W;
+            const P vq = LaneOf<P>::splat(E(0.5) * v1 * inv_dq1);   // walker: 2x face value
+            P Fprev = W.first(y0, y1, y2, y3, y4, S);
 #pragma unroll
             for (int c = 0; c < TQ; ++c) {
                 y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                 y4 = ld(ra + (c + 5) * PW, rb);
                 const P Fn = W.next(y0, y1, y2, y3, y4, S);
                 P d = mul2(sub2(Fprev, Fn), vq);
+                if (JCUR) {
+                    P fc = right ? y2 : y1;
+#pragma unroll
+                    for (int h = 0; h < ROWS; ++h) {
+                        const int cell = (lp + h) * TQ + c;
+                        // (the walker's value is twice the face's)
+                        add_current(cell, 0, pvalid ? double(comp(Fprev, h)) * (0.5 * V1) : 0.0);
+                        add_current(cell, 2, pvalid ? double(comp(fc, h)) * V3 : 0.0);
+                    }
+                }
                 Fprev = Fn;
                 if (BGK) {
                     // the cell itself is the window's y2 (right-moving) or y1
@@ -490,6 +630,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                     d = fma2(sub2(f0, fcell), inv_tau, d);
                 }
                 st(da + c * PW, TQ * PW, d);
+            }
             }
             // the store of chunk k-1 must be done reading the staging tiles
             // before the q2 walkers write them
@@ -507,16 +648,40 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             P y2 = ld(ca + 2 * HX * PW, cb);
             P y3 = ld(ca + 3 * HX * PW, cb);
             P y4 = ld(ca + 4 * HX * PW, cb);
+            P dq[TQ];                                  // flux differences of rows 0..7
+            if constexpr (EXACT) {
+                Weno5Side<double> SX;
+                SX.set(right);
+                ExactWalker WX;
+                double fp = WX.first(y0, y1, y2, y3, y4, right, SX);
+                double Fp = v2 * fp;
+#pragma unroll
+                for (int r = 0; r < TQ; ++r) {
+                    y0 = y1; y1 = y2; y2 = y3; y3 = y4;
+                    y4 = ca[(r + 5) * HX * PW];
+                    const double fn = WX.next(y0, y1, y2, y3, y4, right, SX);
+                    const double Fn = v2 * fn;
+                    dq[r] = div_by(Fn - Fp, a.dq2, inv_dq2);
+                    if (JCUR) add_current(r * TQ + lp, 1, pvalid ? fp * V2 : 0.0);
+                    Fp = Fn;
+                    fp = fn;
+                }
+            } else {
             Walker W;
             P Fprev = W.first(y0, y1, y2, y3, y4, S);
-            P dq[TQ];                                  // flux differences of rows 0..7
 #pragma unroll
             for (int r = 0; r < TQ; ++r) {
                 y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                 y4 = ld(ca + (r + 5) * HX * PW, cb);
                 const P Fn = W.next(y0, y1, y2, y3, y4, S);
                 dq[r] = sub2(Fprev, Fn);
+                if (JCUR)
+#pragma unroll
+                    for (int h = 0; h < ROWS; ++h)
+                        add_current(r * TQ + lp + h, 1,
+                                    pvalid ? double(comp(Fprev, h)) * (0.5 * V2) : 0.0);
                 Fprev = Fn;
+            }
             }
             if (!BX && !failed &&
                 !mbar_wait_bounded(&bars[2 + buf], buf ? phb1 : phb0, a.wait_cycles))
@@ -528,25 +693,64 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             const E* cella = Xb + (HALO * HX + lp + HALO) * PW + lane;
             E* ob1 = o1s + lp * CS;
             E* ob2 = o2s + lp * PW + lane;
-            // FP64 accumulator: element (row r, column lp, p) of chunk k
-            E* accp = static_cast<E*>(a.out2) + ((j0 + Ng) * colstride +
-                                                 (i0 + lp + Ng) * rowstride + xs + k * PW + lane);
+            // element (row r, column lp, p) of chunk k in the outputs that go
+            // from registers to memory, and which of its cells exist
+            const unsigned cell0 = (j0 + Ng) * colstride + (i0 + lp + Ng) * rowstride + xs +
+                                   k * PW + lane;
+            E* accp = static_cast<E*>(a.out2) + cell0;
+            const bool col0 = pvalid && i0 + lp < Nq1, col1 = pvalid && i0 + lp + 1 < Nq1;
 #pragma unroll
             for (int r = 0; r < TQ; ++r) {
                 const P kq = ld(dk + r * TQ * PW, PW);
-                const P kk = fma2(dq[r], vq, kq);
+                P kk;
+                if constexpr (EXACT) {
+                    kk = kq - dq[r];
+                    if (BGK) kk = kk + o2s[(r * TQ + lp) * PW + lane];
+                } else {
+                    kk = fma2(dq[r], vq, kq);
+                }
                 const P fcell = BX ? ld(cella + r * HX * PW, PW) : kk;
-                const P o1 = KOUT ? kk : fma2(kk, c1, BX ? fcell : ld(bb1 + r * TQ * PW, PW));
-                if constexpr (ROWS == 2) {
+                const P b1 = KOUT ? kk : (BX ? fcell : ld(bb1 + r * TQ * PW, PW));
+                P o1;
+                if constexpr (KOUT) o1 = kk;
+                else if constexpr (EXACT) o1 = b1 + kk * c1;
+                else o1 = fma2(kk, c1, b1);
+                if constexpr (ANY) {
+                    // outputs straight from registers, where the cell exists;
+                    // zero in the staging tile elsewhere
+                    const bool row = j0 + r < Nq2;
+                    P o2 = RED2 ? mul2(kk, c2) : o1;
+                    if constexpr (HAS2 && !RED2) {
+                        if constexpr (EXACT) o2 = fcell + kk * c2;
+                        else o2 = fma2(kk, c2, fcell);
+                    }
+#pragma unroll
+                    for (int h = 0; h < ROWS; ++h) {
+                        if (row && (h ? col1 : col0)) {
+                            out1[cell0 + r * colstride + h * rowstride] = comp(o1, h);
+                            // (the accumulator: one add per element and stage)
+                            if (RED2) atomicAdd(accp + r * colstride + h * rowstride, comp(o2, h));
+                            else if (HAS2) accp[r * colstride + h * rowstride] = comp(o2, h);
+                        } else {
+                            comp(o1, h) = E(0);
+                        }
+                    }
+                }
+                if constexpr (ANY && KOUT) {
+                    // k itself: no moments, no images
+                } else if constexpr (ROWS == 2) {
                     ob1[r * TQ * CS + sw0] = o1.x;
                     ob1[r * TQ * CS + CS + sw1] = o1.y;
                 } else {
                     ob1[r * TQ * CS + sw0] = o1;
                 }
+                if constexpr (ANY) continue;
                 if constexpr (RED2 && F64) {
                     // the increment c2 k straight into the accumulator: one
                     // add per element and stage, so acc + inc exactly
                     atomicAdd(accp + r * colstride, mul2(kk, c2));
+                } else if constexpr (HAS2 && EXACT) {
+                    accp[r * colstride] = fcell + kk * c2;     // o2s holds the source term
                 } else if (HAS2) {
                     // QP_X2: the full out2; QP_B1R2: the increment c2 k
                     const P o2 = RED2 ? mul2(kk, c2) : fma2(kk, c2, fcell);
@@ -559,11 +763,18 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
         if (failed) break;
         if (buf) { phx1 ^= 1u; phb1 ^= 1u; } else { phx0 ^= 1u; phb0 ^= 1u; }
         pend &= ~(5u << buf);
-        if (tid == 0) {
+        if (copies) {
+            copy_tiles(k + 2, buf);
+        } else if (ANY) {
+            if (tid == 0) {
+                load_x(k + 2, buf);
+                load_b(k + 2, buf);
+            }
+        } else if (tid == 0) {
             tma_store_3d(&a.tm_o1, o1s, xs + k * PW, i0 + Ng, j0 + Ng);
             if (F64)        // second half of the 32 p (the swizzled rows hold 16)
                 tma_store_3d(&a.tm_o1, o1s + 64 * CS, xs + k * PW + CS, i0 + Ng, j0 + Ng);
-            if (MODE == QP_X2) tma_store_3d(&a.tm_o2, o2s, xs + k * PW, i0 + Ng, j0 + Ng);
+            if (MODE == QP_X2 && !EXACT) tma_store_3d(&a.tm_o2, o2s, xs + k * PW, i0 + Ng, j0 + Ng);
             if (RED2 && !F64) tma_reduce_add_3d(&a.tm_o2, o2s, xs + k * PW, i0 + Ng, j0 + Ng);
             bulk_commit();
             load_x(k + 2, buf);
@@ -573,7 +784,8 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
         // ---- periodic ghost images of border cells, from the staged out1 -------
         // warp w owns tile column w%8; images along q1 (whole column), along q2
         // (rows below g_bot and from g_top) and at the corners (2 N_g <= N_q)
-        if (g_on) {
+        if (g_on && (!ANY || (pvalid && i0 + pc_w < Nq1))) {
+            const int rows = ANY ? min(TQ, Nq2 - j0) : TQ;
             const E* src = o1s + g_src;
             E* dst = out1 + (g_dst + k * PW);
             // q1 / q2 images: this buffer (periodic axis) or the neighbours'
@@ -587,14 +799,14 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                               : dst;
 #pragma unroll
                 for (int r = 0; r < TQ; ++r)
-                    d1[r * (int)colstride + g_d1] = src[r * TQ * CS];
+                    if (!ANY || r < rows) d1[r * (int)colstride + g_d1] = src[r * TQ * CS];
             }
-            for (int r = 0; r < g_bot; ++r) {
+            for (int r = 0; r < min(g_bot, rows); ++r) {
                 const E v = src[r * TQ * CS];
                 dlo[r * (int)colstride + g_d2] = v;
                 if (gc1) dst[r * (int)colstride + gc1 + g_d2] = v;
             }
-            for (int r = g_top; r < TQ; ++r) {
+            for (int r = g_top; r < rows; ++r) {
                 const E v = src[r * TQ * CS];
                 dhi[r * (int)colstride - g_d2] = v;
                 if (gc1) dst[r * (int)colstride + gc1 - g_d2] = v;
@@ -610,13 +822,26 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             load8(c_row, c_ch0, c_key, ov);
             const double o0 = ov[0], o1 = ov[1], o2 = ov[2], o3 = ov[3];
             const double o4 = ov[4], o5 = ov[5], o6 = ov[6], o7 = ov[7];
+            if (ANY && vt_on) {
+                // any N_p1: each value with its own p's velocities
+                const double* v = vtab + buf * 4 * PW + 8 * pc_q;
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    macc[0] += ov[t];
+                    macc[1] = fma(ov[t], v[t], macc[1]);
+                    macc[2] = fma(ov[t], v[PW + t], macc[2]);
+                    macc[3] = fma(ov[t], v[2 * PW + t], macc[3]);
+                    macc[4] = fma(0.5 * ov[t], v[3 * PW + t], macc[4]);
+                }
+                nonfinite |= !isfinite(macc[0]);
+            } else {
             const double S0 = ((o0 + o1) + (o2 + o3)) + ((o4 + o5) + (o6 + o7));
             const double S1 = fma(7.0, o7, fma(6.0, o6, fma(5.0, o5, fma(4.0, o4,
                               fma(3.0, o3, fma(2.0, o2, o1))))));
             const double S2 = fma(49.0, o7, fma(36.0, o6, fma(25.0, o5, fma(16.0, o4,
                               fma(9.0, o3, fma(4.0, o2, o1))))));
             nonfinite |= !isfinite(S0);
-            const double W1 = fma(-t_own, dp1, V1), W2 = V2, W3 = vgrid[Np1 + Np2 + ip3];
+            const double W1 = fma(-t_own, dp1, V1), W2 = V2, W3 = vgrid[Np1 + Np2 + jp3];
             macc[0] += S0;
             macc[1] = fma(W1, S0, fma(dp1, S1, macc[1]));
             macc[2] = fma(W2, S0, macc[2]);
@@ -625,6 +850,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
             const double e0 = fma(W1, W1, fma(W2, W2, W3 * W3));
             const double q = fma(e0, S0, fma(2.0 * W1 * dp1, S1, (dp1 * dp1) * S2));
             macc[4] = fma(0.5, q, macc[4]);
+            }
         }
         ip1 += PW;
         while (ip1 >= Np1) {
@@ -635,6 +861,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     if (failed) {
         // a barrier wait ran out: record it, then let the copies still in
         // flight land (bounded) before the CTA releases its shared memory
+        if (copies) cp_async_wait_everything();
         if (warp == 0) bulk_wait_all();
         if (tid == 0) {
             atomicExch(a.err, 4);
@@ -663,32 +890,51 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
 #pragma unroll
             for (int h = 0; h < NQUART; ++h) v += red[(h * NQ + cq) * kNumMom + q];
             const int ii = i0 + (cq & 7), jj = j0 + (cq >> 3);
-            a.mom_out[(((long long)split * kNumMom + q) * a.Ns + s) * plane
-                      + (long long)jj * Nq1 + ii] = v;
+            if (!ANY || (ii < Nq1 && jj < Nq2))
+                a.mom_out[(((long long)split * kNumMom + q) * a.Ns + s) * plane
+                          + (long long)jj * Nq1 + ii] = v;
+        }
+    }
+    if (JCUR) {
+        // currents of this split (every warp is past the chunks' last barrier)
+        for (int c = tid; c < NQ * 3; c += NT) {
+            const int cell = c / 3, q = c % 3;
+            const int ii = i0 + (cell & 7), jj = j0 + (cell >> 3);
+            if (ii < Nq1 && jj < Nq2)
+                a.j_out[(((long long)split * 3 + q) * a.Ns + s) * plane +
+                        (long long)jj * Nq1 + ii] = jacc[c];
         }
     }
 }
 
-template <typename E, int R, int W>
+template <typename E, int R, int W, bool X, int G>
 static void (*pick_qpair(int bgk, int mode))(QStageArgs) {
-    switch (mode) {
-        case QP_X1:
-            return bgk ? qpair_kernel<E, true, QP_X1, R, W> : qpair_kernel<E, false, QP_X1, R, W>;
-        case QP_X2:
-            return bgk ? qpair_kernel<E, true, QP_X2, R, W> : qpair_kernel<E, false, QP_X2, R, W>;
-        case QP_B1:
-            return bgk ? qpair_kernel<E, true, QP_B1, R, W> : qpair_kernel<E, false, QP_B1, R, W>;
-        case QP_K:
-            return bgk ? qpair_kernel<E, true, QP_K, R, W> : qpair_kernel<E, false, QP_K, R, W>;
-        default:
-            return bgk ? qpair_kernel<E, true, QP_B1R2, R, W>
-                       : qpair_kernel<E, false, QP_B1R2, R, W>;
+    if constexpr (G == QG_CURRENTS) {
+        return bgk ? qpair_kernel<E, true, QP_K, R, W, X, G> : qpair_kernel<E, false, QP_K, R, W, X, G>;
+    } else {
+        switch (mode) {
+            case QP_X1:
+                return bgk ? qpair_kernel<E, true, QP_X1, R, W, X, G>
+                           : qpair_kernel<E, false, QP_X1, R, W, X, G>;
+            case QP_X2:
+                return bgk ? qpair_kernel<E, true, QP_X2, R, W, X, G>
+                           : qpair_kernel<E, false, QP_X2, R, W, X, G>;
+            case QP_B1:
+                return bgk ? qpair_kernel<E, true, QP_B1, R, W, X, G>
+                           : qpair_kernel<E, false, QP_B1, R, W, X, G>;
+            case QP_K:
+                return bgk ? qpair_kernel<E, true, QP_K, R, W, X, G>
+                           : qpair_kernel<E, false, QP_K, R, W, X, G>;
+            default:
+                return bgk ? qpair_kernel<E, true, QP_B1R2, R, W, X, G>
+                           : qpair_kernel<E, false, QP_B1R2, R, W, X, G>;
+        }
     }
 }
 
 // the stage mode from which buffers the stage reads and writes, then the
 // reconstruction's instantiation
-template <typename E>
+template <typename E, bool X, int G>
 static cudaError_t launch_qpair(const QStageArgs& a, int bgk, int recon, dim3 grid, size_t smem,
                                 cudaStream_t st) {
     const bool has2 = a.out2 != nullptr;
@@ -700,20 +946,29 @@ static cudaError_t launch_qpair(const QStageArgs& a, int bgk, int recon, dim3 gr
     else if (!has2) mode = QP_B1;
     else if (a.base2 == a.out2) mode = QP_B1R2;
     else return cudaErrorInvalidValue;        // excluded by the host's dispatch
+    if (G == QG_CURRENTS && mode != QP_K) return cudaErrorInvalidValue;
     // FP32: row pairs, 8 warps, 2 CTAs per SM; FP64: one row per thread, 16
     // warps, 1 CTA per SM (the shared memory of the double-buffered tiles)
     constexpr int W = sizeof(E) == 4 ? 2 : 1;
     void (*k)(QStageArgs);
     switch (recon) {
-        case BOLT_RECON_MINMOD: k = pick_qpair<E, BOLT_RECON_MINMOD, W>(bgk, mode); break;
-        case BOLT_RECON_PPM: k = pick_qpair<E, BOLT_RECON_PPM, W>(bgk, mode); break;
-        case BOLT_RECON_PC: k = pick_qpair<E, BOLT_RECON_PC, W>(bgk, mode); break;
-        default: k = pick_qpair<E, BOLT_RECON_WENO5, W>(bgk, mode); break;
+        case BOLT_RECON_MINMOD: k = pick_qpair<E, BOLT_RECON_MINMOD, W, X, G>(bgk, mode); break;
+        case BOLT_RECON_PPM: k = pick_qpair<E, BOLT_RECON_PPM, W, X, G>(bgk, mode); break;
+        case BOLT_RECON_PC: k = pick_qpair<E, BOLT_RECON_PC, W, X, G>(bgk, mode); break;
+        default: k = pick_qpair<E, BOLT_RECON_WENO5, W, X, G>(bgk, mode); break;
     }
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k<<<grid, W == 2 ? NTHREADS : 2 * NTHREADS, smem, st>>>(a);
     return cudaGetLastError();
+}
+
+// the kernels for any grid, with or without currents
+template <typename E, bool X>
+static cudaError_t launch_qpair_any(const QStageArgs& a, int bgk, int recon, dim3 grid,
+                                    size_t smem, cudaStream_t st) {
+    return a.want_j ? launch_qpair<E, X, QG_CURRENTS>(a, bgk, recon, grid, smem, st)
+                    : launch_qpair<E, X, QG_ANY>(a, bgk, recon, grid, smem, st);
 }
 
 }  // namespace bolt
