@@ -122,6 +122,8 @@ struct BoltCtx {
     int timing_on, timing_depth;
     int pair_enabled;       // paired kernel allowed (BOLT_NO_PAIR unset)
     PShape pshape;          // launch shape of the p-stage kernel
+    int line_ok;            // 1D1V, periodic in q2: the line kernel's grids
+    LineShape line;
     int pair_shape_ok;      // grid/method meet the paired kernel's shape conditions
     int any_shape_ok;       // ... or those of its form for any grid
 };
@@ -317,6 +319,14 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         const int nchunks = (ctx->Np + PW - 1) / PW;
         const long long base_ctas = (long long)ctx->ntiles1 * ctx->ntiles2 * g.N_s;
         PSplit sp = choose_psplit(nchunks, base_ctas, current_sm_count(), smem_est);
+        ctx->line_ok = g.N_q2 == 1 && p.bc_q2 == BOLT_BC_PERIODIC && g.N_p2 == 1 && g.N_p3 == 1;
+        if (ctx->line_ok) {
+            ctx->line = choose_line(g.N_q1, g.N_s, ctx->Np, current_sm_count());
+            if (!p.fields_enabled) {
+                sp.chunks_per_split = ctx->line.chunks_per_split;
+                sp.nsplit = (nchunks + sp.chunks_per_split - 1) / sp.chunks_per_split;
+            }
+        }
         // BOLT_CHUNKS_PER_SPLIT fixes the split instead (tests run one problem
         // under several splits; results differ only in the order of the FP64
         // moment partial sums)
@@ -329,6 +339,8 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         }
         ctx->chunks_per_split = sp.chunks_per_split;
         ctx->nsplit = sp.nsplit;
+        if (ctx->line_ok && ctx->line.threads > sp.chunks_per_split * PW)
+            ctx->line.threads = sp.chunks_per_split * PW;
     }
     const size_t rowbytes = (size_t)g.N_s * ctx->Np * ctx->elem;
     ctx->use_tma_ok = (g.N_ghost >= HALO) && (rowbytes % 16 == 0) &&
@@ -835,8 +847,14 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
                                     : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk,
                                                   ctx->bgk_direct, ctx->ntab);
     const int bgk = ctx->bgk, recon = ctx->recon_q;
+    // 1D1V: the line kernel, except for currents (q2 faces) and for
+    // bolt_dfdt without fields (as above)
+    const bool line = ctx->line_ok && !want_j && (!write_k || ctx->p.fields_enabled);
     cudaError_t e;
-    if (pair)
+    if (line)
+        e = ctx->elem == 4 ? launch_line_f32(a, recon, bgk, ctx->line, st)
+                           : launch_line_f64(a, recon, bgk, ctx->line, st);
+    else if (pair)
         e = ctx->elem == 4 ? launch_qpair_f32(a, bgk, recon, grid, smem, st)
             : ctx->p.dtype == BOLT_F64_FAST
                 ? launch_qpair_f64(a, bgk, recon, grid, smem, st)

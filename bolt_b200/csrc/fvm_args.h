@@ -198,6 +198,7 @@ struct PStageArgs {
 };
 
 constexpr int PTHREADS_MAX = 512;
+constexpr int LINE_THREADS = 256;       // 1D1V q-stage: most p-threads per CTA
 
 // elements from one p1 row of the p-stage's shared-memory blocks to the next:
 // odd, so that lanes walking neighbouring rows read distinct banks

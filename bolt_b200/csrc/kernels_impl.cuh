@@ -5,6 +5,7 @@
 #include "launch.h"
 #include "fvm_kernels.cuh"
 #include "pstage_kernel.cuh"
+#include "line_kernel.cuh"
 #include "asl_kernels.cuh"
 
 namespace bolt {
@@ -43,6 +44,35 @@ cudaError_t BOLT_CAT(launch_qstage_, BOLT_SUFFIX)(const QStageArgs& a, int recon
         case BOLT_RECON_MINMOD: return qdispatch<BOLT_RECON_MINMOD>(a, tiling, bgk, grid, smem, st);
         case BOLT_RECON_PPM: return qdispatch<BOLT_RECON_PPM>(a, tiling, bgk, grid, smem, st);
         default: return qdispatch<BOLT_RECON_WENO5>(a, tiling, bgk, grid, smem, st);
+    }
+}
+
+template <int RECON, bool BGK>
+static void (*pick_line(int r))(QStageArgs) {
+    switch (r) {
+        case 1: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 1>;
+        case 2: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 2>;
+        case 4: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 4>;
+        default: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 8>;
+    }
+}
+
+template <int RECON>
+static cudaError_t lline(const QStageArgs& a, int bgk, const LineShape& shape, cudaStream_t st) {
+    void (*k)(QStageArgs) = bgk ? pick_line<RECON, true>(shape.r)
+                                : pick_line<RECON, false>(shape.r);
+    const dim3 grid((a.Nq1 + shape.r - 1) / shape.r, a.Ns * a.nsplit);
+    k<<<grid, shape.threads + (bgk ? 32 : 0), 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t BOLT_CAT(launch_line_, BOLT_SUFFIX)(const QStageArgs& a, int recon, int bgk,
+                                                const LineShape& shape, cudaStream_t st) {
+    switch (recon) {
+        case BOLT_RECON_PC: return lline<BOLT_RECON_PC>(a, bgk, shape, st);
+        case BOLT_RECON_MINMOD: return lline<BOLT_RECON_MINMOD>(a, bgk, shape, st);
+        case BOLT_RECON_PPM: return lline<BOLT_RECON_PPM>(a, bgk, shape, st);
+        default: return lline<BOLT_RECON_WENO5>(a, bgk, shape, st);
     }
 }
 

@@ -63,6 +63,30 @@ inline PSplit choose_psplit(int nchunks, long long base_ctas, int sms, size_t sm
     return PSplit{(nchunks + best_cps - 1) / best_cps, best_cps};
 }
 
+// Launch shape of the 1D1V q-stage (line_kernel): q-cells per thread, p-threads
+// per CTA, p-chunks of 32 per CTA.  R grows while the threads still fill about
+// two warps per scheduler; the p-range of a q-cell is split over CTAs only while
+// there are fewer than two CTAs per SM (each split is one more slot for the next
+// stage's prologue to sum).
+struct LineShape {
+    int r, threads, chunks_per_split;
+};
+
+inline LineShape choose_line(int Nq1, int Ns, int Np, int sms) {
+    LineShape L;
+    const long long cells = (long long)Nq1 * Ns * Np;
+    L.r = 1;
+    while (L.r < 8 && cells / (2 * L.r) >= (long long)sms * 256) L.r *= 2;
+    L.threads = Np >= LINE_THREADS ? LINE_THREADS : (Np + 31) / 32 * 32;
+    const int chunks = (Np + PW - 1) / PW, per_cta = L.threads / PW;
+    const long long ctas = (long long)((Nq1 + L.r - 1) / L.r) * Ns;
+    long long splits = (2LL * sms + ctas - 1) / ctas;
+    const long long most = (chunks + per_cta - 1) / per_cta;
+    if (splits > most) splits = most;
+    L.chunks_per_split = (int)((chunks + splits - 1) / splits);
+    return L;
+}
+
 // SM count of the current device (148 on B200 if the query fails)
 inline int current_sm_count() {
     int dev = 0, sms = 148;
@@ -134,6 +158,8 @@ inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, long long ctas,
 #define BOLT_DECLARE_LAUNCHERS(SUFFIX, T)                                                   \
     cudaError_t launch_qstage_##SUFFIX(const QStageArgs& a, int recon, int tiling, int bgk, \
                                        dim3 grid, size_t smem, cudaStream_t st);            \
+    cudaError_t launch_line_##SUFFIX(const QStageArgs& a, int recon, int bgk,               \
+                                     const LineShape& shape, cudaStream_t st);              \
     cudaError_t launch_pstage_##SUFFIX(const PStageArgs& a, int recon, dim3 grid,           \
                                        int threads, size_t smem, cudaStream_t st);          \
     cudaError_t launch_moment_##SUFFIX(const void* f, int mid, double* out, int Ns,          \
