@@ -171,6 +171,15 @@ struct AslArgs {
     SpeciesGrid sg;
 };
 
+// shared memory of the fused source step: the p-block, then (8-byte aligned)
+// two factor tables and the p-cell centres
+__host__ __device__ inline unsigned asl_block_bytes(int Np, unsigned elem) {
+    return ((unsigned)Np * elem + 15u) & ~15u;
+}
+__host__ __device__ inline unsigned asl_source_smem(int Np, int ntab, unsigned elem) {
+    return asl_block_bytes(Np, elem) + 3u * (unsigned)ntab * 8u;
+}
+
 struct PStageArgs {
     const void* fs;        // stage input (ghosted)
     const void* kq;        // q-part of df/dt (ghosted layout, interior valid)

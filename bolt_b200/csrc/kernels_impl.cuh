@@ -159,4 +159,15 @@ cudaError_t BOLT_CAT(launch_asl_src_, BOLT_SUFFIX)(const QStageArgs& a, const vo
     return cudaGetLastError();
 }
 
+cudaError_t BOLT_CAT(launch_asl_source_, BOLT_SUFFIX)(const QStageArgs& a, const void* in,
+                                                      void* out, double dt, int* flag,
+                                                      cudaStream_t st) {
+    auto k = asl_source_kernel<BOLT_T>;
+    const unsigned smem = asl_source_smem(a.Np, a.Np1 + a.Np2 + a.Np3, sizeof(BOLT_T));
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(a.Nq1 * a.Nq2, a.Ns), 256, smem, st>>>(a, in, out, dt, flag);
+    return cudaGetLastError();
+}
+
 }  // namespace bolt

@@ -203,6 +203,12 @@ cudaError_t launch_asl_src_f64(const QStageArgs& a, const void* in, const void* 
 cudaError_t launch_asl_src_f32(const QStageArgs& a, const void* in, const void* base, void* out,
                                double c, int mode, int* flag, double* mom_out, cudaStream_t st);
 
+// the whole RK2 step of the source, the p-block in shared memory
+cudaError_t launch_asl_source_f64(const QStageArgs& a, const void* in, void* out, double dt,
+                                  int* flag, cudaStream_t st);
+cudaError_t launch_asl_source_f32(const QStageArgs& a, const void* in, void* out, double dt,
+                                  int* flag, cudaStream_t st);
+
 // paired q-stage (8x8 tiling, fused combine, TMA in and out): FP32, and FP64
 // with FMA contraction and Newton-refined reciprocals (BOLT_F64_FAST)
 cudaError_t launch_qpair_f32(const QStageArgs& a, int bgk, int recon, dim3 grid, size_t smem,
