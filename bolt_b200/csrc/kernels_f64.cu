@@ -21,6 +21,11 @@ cudaError_t launch_field_halo(const FieldArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_fdtd(const FieldArgs& a, cudaStream_t st, long long* launches) {
+    if (a.Nq1g * a.Nq2g <= kFieldClusterCells) {
+        fdtd_step_kernel<<<kFieldCluster, kFieldThreads, 0, st>>>(a);
+        if (launches) *launches += 1;
+        return cudaGetLastError();
+    }
     for (int part = 0; part < 3; ++part) {
         const cudaError_t e = launch_fdtd_part(a, part, st, launches);
         if (e != cudaSuccess) return e;
