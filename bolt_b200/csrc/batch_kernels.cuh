@@ -22,6 +22,12 @@
 //   * out1 = base1 + c1 dt k, out2 = base2 + c2 dt k (RK4 stage combine,
 //     integrators.py:15-28), periodic ghost images of out1, FP64 moments of
 //     out1 accumulated per thread across chunks, non-finite check.
+//
+// What bounds it: instruction issue and the latency of the loads (the working
+// set of the 256-run sweep fits L2): 81 us per stage of 10.9M cells (99 us with
+// the three-weight faces and the reduction of the exponent in v - u).  Eight
+// cells per warp as f32x2 pairs gave 86 us, and the same without shared memory
+// 90 us and up to 30 % more on batches of tens of runs.
 #pragma once
 
 #include "fvm_args.h"
@@ -61,24 +67,27 @@ struct BatchStageArgs {
     int source;            // BGK on
 };
 
-// e^x to FP32 accuracy: Cody-Waite reduction x = n ln2 + r, |r| <= ln2/2, in
-// FP64, then 2^(r/ln2) by the hardware base-2 exponential (ex2.approx,
-// relative error ~2^-22) scaled by 2^n built from its exponent bits.  Results
-// below the FP32 normal range are flushed to zero, above it are infinite.
-__device__ __forceinline__ float batch_exp(double x) {
-    if (x < -87.0) return 0.0f;
-    if (x > 88.0) return __int_as_float(0x7f800000);
-    const double log2e = 1.4426950408889634, ln2 = 0.6931471805599453;
-    const double n = rint(x * log2e);
-    const double r = fma(-n, ln2, x);
+// 2^x to FP32 accuracy for FP64 x: the integer part by adding 1.5 * 2^52 (its
+// low word is the integer), the rest, |r| <= 1/2, by the hardware base-2
+// exponential (ex2.approx, relative error ~2^-22), scaled by 2^n built from its
+// exponent bits.  Results below the FP32 normal range are flushed to zero, above
+// it are infinite; a NaN stays one.
+__device__ __forceinline__ float batch_exp2(double x) {
+    x = x < -160.0 ? -160.0 : (x > 160.0 ? 160.0 : x);
+    const double magic = 6755399441055744.0;
+    const double t = x + magic;
+    const float r = float(x - (t - magic));
     float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(float(r * log2e)));
-    return e * __int_as_float((int(n) + 127) << 23);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(r));
+    const int n = min(max(__double2loint(t) + 127, 0), 255);
+    return e * __int_as_float(n << 23);
 }
 
 // Maxwellian parameters of one q-cell from its raw moment sums
 // (collision_operator.py:102-118, f0 :49-65 with p_dim = 1):
-// {n A, u1, -m / (2 kB T)}
+// {n A, c0, c1, c2} with f0(v) = n A 2^(c0 + c1 v + c2 v^2), the exponent
+// -m (v - u1)^2 / (2 kB T) expanded in v (FP64: its terms cancel to ~1e-13 at
+// the widest grids, against 2^-22 of the exponential)
 __device__ __forceinline__ void batch_maxwell(const BatchRunDev& R, const double* mm,
                                               double* out) {
     const double eps = 1e-30;
@@ -93,9 +102,11 @@ __device__ __forceinline__ void batch_maxwell(const BatchRunDev& R, const double
                      / (n + eps) + eps;                     // (1/p_dim) with p_dim = 1
     const double twokT = (2.0 * kB) * T;
     const double A = sqrt(m / ((2.0 * 3.141592653589793 * kB) * T));
+    const double b = -m / twokT * 1.4426950408889634;      // log2 e
     out[0] = n * A;
-    out[1] = u1;
-    out[2] = -m / twokT;
+    out[1] = b * u1 * u1;
+    out[2] = -2.0 * b * u1;
+    out[3] = b;
 }
 
 __device__ __forceinline__ void batch_moments_out(const BatchRunDev& R, double m0, double m1,
@@ -113,7 +124,7 @@ batch_stage_kernel(const BatchStageArgs a) {
     constexpr int TQ = NW * kBatchCellsPerWarp;
     constexpr int ROWS = TQ + 2 * kBatchNg;
     __shared__ float X[2][ROWS][PW];      // chunk c in X[c & 1]; chunk c+1 loads meanwhile
-    __shared__ double par[TQ][3];
+    __shared__ double par[TQ][4];
     __shared__ int item_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     bool nonfinite = false;
@@ -167,39 +178,42 @@ batch_stage_kernel(const BatchStageArgs a) {
                 const double V = R.p1_start + (0.5 + p) * R.dp1;
                 const float v = float(V);
                 const bool right = v > 0.0f;
-                Weno5Side<float> S;
+                const double Vh = 0.5 * V * V;
+                Weno5PairT<float, float> S;
                 S.set(right);
-                Weno5Walker<false, float> W;
+                Weno5PairWalkerT<float, float> W;      // returns twice the face value
+                const float vq = 0.5f * v * inv_dq;
                 const float (*Xb)[PW] = X[b];
                 // the combine bases of this warp's 4 cells, loaded before the
                 // stencil so that their latency overlaps it
+                const long long o0 = R.f_off + (long long)(i0 + j0 + kBatchNg) * Np1 + p;
                 float b1v[4], b2v[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const long long o = R.f_off + (long long)(i0 + j0 + q + kBatchNg) * Np1 + p;
-                    b1v[q] = a.base1[o];
-                    b2v[q] = a.out2 ? a.base2[o] : 0.0f;
+                    b1v[q] = a.base1[o0 + q * Np1];
+                    b2v[q] = a.out2 ? a.base2[o0 + q * Np1] : 0.0f;
                 }
                 // face between local cells f and f+1 reads rows f+1+off .. f+5+off
                 const int r0 = j0 + (right ? 0 : 1);
                 float y0 = Xb[r0][lane], y1 = Xb[r0 + 1][lane], y2 = Xb[r0 + 2][lane];
                 float y3 = Xb[r0 + 3][lane], y4 = Xb[r0 + 4][lane];
-                float Fprev = v * W.first(y0, y1, y2, y3, y4, right, S);
+                float Fprev = W.first(y0, y1, y2, y3, y4, S);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int j = j0 + q;             // local cell
                     y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                     y4 = Xb[r0 + 5 + q][lane];
-                    const float Fn = v * W.next(y0, y1, y2, y3, y4, right, S);
-                    float k = (Fprev - Fn) * inv_dq;
+                    const float Fn = W.next(y0, y1, y2, y3, y4, S);
+                    float k = (Fprev - Fn) * vq;
                     Fprev = Fn;
-                    const float fc = Xb[j + kBatchNg][lane];
+                    // the cell itself is the window's y2 (right-moving) or y1
+                    const float fc = right ? y2 : y1;
                     if (a.source) {
-                        const double dv = V - par[j][1];
-                        const float f0 = float(par[j][0]) * batch_exp(par[j][2] * (dv * dv));
+                        const double* m = par[j];
+                        const float f0 = float(m[0]) * batch_exp2(fma(V, fma(V, m[3], m[2]), m[1]));
                         k = fmaf(f0 - fc, inv_tau, k);
                     }
-                    const long long o = R.f_off + (long long)(i0 + j + kBatchNg) * Np1 + p;
+                    const long long o = o0 + q * Np1;
                     const float o1 = fmaf(k, c1, b1v[q]);
                     a.out1[o] = o1;
                     if (a.out2) a.out2[o] = fmaf(k, c2, b2v[q]);
@@ -211,7 +225,7 @@ batch_stage_kernel(const BatchStageArgs a) {
                     const double od = o1;
                     acc[q][0] += od;
                     acc[q][1] = fma(od, V, acc[q][1]);
-                    acc[q][2] = fma(0.5 * od, V * V, acc[q][2]);
+                    acc[q][2] = fma(od, Vh, acc[q][2]);
                 }
             }
             __syncthreads();                      // X[b] reads done before it is refilled
