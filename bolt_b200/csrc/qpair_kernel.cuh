@@ -47,8 +47,8 @@
 // the out2 staging tile, and a second output that is stored (first RK4 stage)
 // goes from the q2 walkers' registers to memory.  The scalar kernel (8 warps,
 // four divisions a face, single-buffered halo) left the FP64 pipe idle most of
-// the time: an RK4 step of 64^2 x 24^3 cells took 9.62 ms, here 3.78 ms (its
-// bytes alone 1.2 ms); what bounds it now is the latency of the dependent FP64
+// the time: an RK4 step of 64^2 x 24^3 cells took 9.62 ms, here 3.59 ms (its
+// bytes alone 1.2 ms; 3.78 ms with the q1 walk rolled); what bounds it now is the latency of the dependent FP64
 // chains at 16 warps per SM.
 //
 // QG_ANY, QG_CURRENTS: any grid.  The halo and base tiles come by TMA where rows
@@ -583,7 +583,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                 double fp = WX.first(y0, y1, y2, y3, y4, right, SX);
                 double Fp = v1 * fp;
                 double* db = o2s + lp * TQ * PW + lane;
-#pragma unroll 1
+#pragma unroll
                 for (int c = 0; c < TQ; ++c) {
                     y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                     y4 = ra[(c + 5) * PW];
