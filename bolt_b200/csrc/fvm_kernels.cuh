@@ -574,6 +574,36 @@ qstage_kernel(const __grid_constant__ QStageArgs a) {
     }
 }
 
+// (i1, i2, i3) of a p-cell index that a thread advances by a fixed stride,
+// kept without divisions: the stride is split once into its p1 remainder and
+// its p2 / p3 row steps, and each advance carries from p1 into p2 and from p2
+// into p3 (each part stays below twice its range, so one subtraction does)
+struct PCellWalk {
+    int i1, i2, i3;        // current p-cell
+    int d1, d2, d3;        // the stride as (p1, p2, p3) steps
+    int Np1, Np2;
+    __device__ __forceinline__ PCellWalk(int p, int stride, int np1, int np2)
+        : Np1(np1), Np2(np2) {
+        i1 = p % np1;
+        const int r = p / np1;
+        i2 = r % np2;
+        i3 = r / np2;
+        d1 = stride % np1;
+        const int rs = stride / np1;
+        d2 = rs % np2;
+        d3 = rs / np2;
+    }
+    __device__ __forceinline__ void advance() {
+        i1 += d1;
+        int c = 0;
+        if (i1 >= Np1) { i1 -= Np1; c = 1; }
+        i2 += d2 + c;
+        c = 0;
+        if (i2 >= Np2) { i2 -= Np2; c = 1; }
+        i3 += d3 + c;
+    }
+};
+
 // ---------------------------------------------------------------------------
 // moments (compute_moments.py:7-59 with moments.py:6-58), FP64 output.
 // One CTA per (ghosted q-cell, species).
@@ -587,9 +617,9 @@ moment_kernel(const T* f, int mid, double* out, int Ns, int Np1, int Np2, int Np
     const int Np = Np1 * Np2 * Np3;
     const T* fp = f + ((long long)q * Ns + s) * Np;
     double acc = 0.0;
-    for (int c = tid; c < Np; c += 256) {
-        const int i1 = c % Np1, i2 = (c / Np1) % Np2, i3 = c / (Np1 * Np2);
-        const PVel V = lane_velocity(sg, s, i1, i2, i3);
+    PCellWalk w(tid, 256, Np1, Np2);
+    for (int c = tid; c < Np; c += 256, w.advance()) {
+        const PVel V = lane_velocity(sg, s, w.i1, w.i2, w.i3);
         const double fv = double(fp[c]);
         double g;
         switch (mid) {
@@ -651,36 +681,6 @@ __device__ __forceinline__ void add_moment_run(const double (&o)[n], double V1, 
     const double e0 = fma(V1, V1, fma(v2, v2, v3 * v3));
     acc[4] = fma(0.5, fma(e0, S0, fma(2.0 * V1 * dp1, S1, (dp1 * dp1) * S2)), acc[4]);
 }
-
-// (i1, i2, i3) of a p-cell index that a thread advances by a fixed stride,
-// kept without divisions: the stride is split once into its p1 remainder and
-// its p2 / p3 row steps, and each advance carries from p1 into p2 and from p2
-// into p3 (each part stays below twice its range, so one subtraction does)
-struct PCellWalk {
-    int i1, i2, i3;        // current p-cell
-    int d1, d2, d3;        // the stride as (p1, p2, p3) steps
-    int Np1, Np2;
-    __device__ __forceinline__ PCellWalk(int p, int stride, int np1, int np2)
-        : Np1(np1), Np2(np2) {
-        i1 = p % np1;
-        const int r = p / np1;
-        i2 = r % np2;
-        i3 = r / np2;
-        d1 = stride % np1;
-        const int rs = stride / np1;
-        d2 = rs % np2;
-        d3 = rs / np2;
-    }
-    __device__ __forceinline__ void advance() {
-        i1 += d1;
-        int c = 0;
-        if (i1 >= Np1) { i1 -= Np1; c = 1; }
-        i2 += d2 + c;
-        c = 0;
-        if (i2 >= Np2) { i2 -= Np2; c = 1; }
-        i3 += d3 + c;
-    }
-};
 
 // The five BGK moments of the interior cells as one "split" of partial sums
 // ([1][5][Ns][Nq2][Nq1], sums without the measure factor).  One CTA per q-cell
@@ -876,29 +876,33 @@ ghost_kernel(T* f, const T* dl, const T* dr, const T* db, const T* dt,
         // corner ghost takes the q1 map of the q2 map of its own p2 index.
         // Then the Dirichlet inflow values where the velocity normal to the
         // edge points into the domain.
-        for (int sp = tid; sp < rowlen; sp += nt) {
-            const int p = sp % Np;
-            const int i1 = p % Np1, i2 = (p / Np1) % Np2;
-            int ps = sp, k2 = i2;                          // source p2 index
-            if (m2) k2 = Np2 - 1 - k2;
-            if (m1) {
-                if (sg.polar2d) {
-                    const int H = Np2 / 2;
-                    k2 = k2 < H ? H - 1 - k2 : Np2 - 1 + H - k2;
-                } else {
-                    ps += Np1 - 1 - 2 * i1;
+        // (indices kept by a walker instead of divisions of an index per value)
+        for (int s = 0; s < Ns; ++s) {
+            PCellWalk w(tid, nt, Np1, Np2);
+            for (int p = tid; p < Np; p += nt, w.advance()) {
+                const int sp = s * Np + p;
+                int ps = sp, k2 = w.i2;                    // source p2 index
+                if (m2) k2 = Np2 - 1 - k2;
+                if (m1) {
+                    if (sg.polar2d) {
+                        const int H = Np2 / 2;
+                        k2 = k2 < H ? H - 1 - k2 : Np2 - 1 + H - k2;
+                    } else {
+                        ps += Np1 - 1 - 2 * w.i1;
+                    }
                 }
+                ps += Np1 * (k2 - w.i2);
+                T v = have ? src[ps] : T(0);
+                if (d1 || d2) {
+                    const double v1 = sg.p1_start[s] + (0.5 + w.i1) * sg.dp1[s];
+                    const double v2 = sg.p2_start[s] + (0.5 + w.i2) * sg.dp2[s];
+                    if (d1 && i < 0 && v1 > 0) v = dl[g + sp];
+                    if (d1 && i >= Nq1 && v1 < 0) v = dr[g + sp];
+                    if (d2 && j < 0 && v2 > 0) v = db[g + sp];
+                    if (d2 && j >= Nq2 && v2 < 0) v = dt[g + sp];
+                }
+                dst[sp] = v;
             }
-            ps += Np1 * (k2 - i2);
-            T v = have ? src[ps] : T(0);
-            const int s = sp / Np;
-            const double v1 = sg.p1_start[s] + (0.5 + i1) * sg.dp1[s];
-            const double v2 = sg.p2_start[s] + (0.5 + i2) * sg.dp2[s];
-            if (d1 && i < 0 && v1 > 0) v = dl[g + sp];
-            if (d1 && i >= Nq1 && v1 < 0) v = dr[g + sp];
-            if (d2 && j < 0 && v2 > 0) v = db[g + sp];
-            if (d2 && j >= Nq2 && v2 < 0) v = dt[g + sp];
-            dst[sp] = v;
         }
     }
 }
