@@ -24,6 +24,16 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 __device__ __forceinline__ int wrapi(int x, int n) { return ((x % n) + n) % n; }
+// the circular neighbours of x in 0 .. n - 1
+__device__ __forceinline__ int up(int x, int n) { return x + 1 == n ? 0 : x + 1; }
+__device__ __forceinline__ int down(int x, int n) { return x == 0 ? n - 1 : x - 1; }
+
+// a/b from r = 1/b (the spacings and eps are the same for every cell), an infinite
+// quotient as the division gives it
+__device__ __forceinline__ double field_div(double a, double b, double r) {
+    const double q = a * r;
+    return fabs(q) < INFINITY ? fma(fma(-b, q, a), r, q) : q;
+}
 
 // J from partial sums (or the caller's J); copy of the cell-centred E before the update
 __device__ __forceinline__ void fdtd_prepare(const FieldArgs& a, int first, int step) {
@@ -77,16 +87,21 @@ __device__ __forceinline__ void fdtd_e(const FieldArgs& a, int first, int step) 
     const double* B2 = a.yee + 4 * n;
     const double* B3 = a.yee + 5 * n;
     const double cf = a.dt / (a.mu * a.eps);
+    const double r1 = 1.0 / a.dq1, r2 = 1.0 / a.dq2, re = 1.0 / a.eps;
     for (int t = first; t < n; t += step) {
         const int g1 = t % a.Nq1g, g2 = t / a.Nq1g;
-        const int p1 = g2 * a.Nq1g + wrapi(g1 + 1, a.Nq1g);     // shift(.., -1, 0)
-        const int p2 = wrapi(g2 + 1, a.Nq2g) * a.Nq1g + g1;     // shift(.., 0, -1)
-        const double curl1 = (B3[p2] - B3[t]) / a.dq2;
-        const double curl2 = -(B3[p1] - B3[t]) / a.dq1;
-        const double curl3 = (B2[p1] - B2[t]) / a.dq1 - (B1[p2] - B1[t]) / a.dq2;
-        a.yee[0 * n + t] = a.yee[0 * n + t] + (cf * curl1 - (a.J[0 * n + t] * a.dt) / a.eps);
-        a.yee[1 * n + t] = a.yee[1 * n + t] + (cf * curl2 - (a.J[1 * n + t] * a.dt) / a.eps);
-        a.yee[2 * n + t] = a.yee[2 * n + t] + (cf * curl3 - (a.J[2 * n + t] * a.dt) / a.eps);
+        const int p1 = g2 * a.Nq1g + up(g1, a.Nq1g);     // shift(.., -1, 0)
+        const int p2 = up(g2, a.Nq2g) * a.Nq1g + g1;     // shift(.., 0, -1)
+        const double curl1 = field_div(B3[p2] - B3[t], a.dq2, r2);
+        const double curl2 = field_div(-(B3[p1] - B3[t]), a.dq1, r1);
+        const double curl3 = field_div(B2[p1] - B2[t], a.dq1, r1) -
+                             field_div(B1[p2] - B1[t], a.dq2, r2);
+        a.yee[0 * n + t] = a.yee[0 * n + t] +
+                           (cf * curl1 - field_div(a.J[0 * n + t] * a.dt, a.eps, re));
+        a.yee[1 * n + t] = a.yee[1 * n + t] +
+                           (cf * curl2 - field_div(a.J[1 * n + t] * a.dt, a.eps, re));
+        a.yee[2 * n + t] = a.yee[2 * n + t] +
+                           (cf * curl3 - field_div(a.J[2 * n + t] * a.dt, a.eps, re));
     }
 }
 
@@ -96,13 +111,15 @@ __device__ __forceinline__ void fdtd_b(const FieldArgs& a, int first, int step) 
     const double* E1 = a.yee;
     const double* E2 = a.yee + n;
     const double* E3 = a.yee + 2 * n;
+    const double r1 = 1.0 / a.dq1, r2 = 1.0 / a.dq2;
     for (int t = first; t < n; t += step) {
         const int g1 = t % a.Nq1g, g2 = t / a.Nq1g;
-        const int m1 = g2 * a.Nq1g + wrapi(g1 - 1, a.Nq1g);     // shift(.., 1, 0)
-        const int m2 = wrapi(g2 - 1, a.Nq2g) * a.Nq1g + g1;     // shift(.., 0, 1)
-        const double curl1 = (E3[t] - E3[m2]) / a.dq2;
-        const double curl2 = -(E3[t] - E3[m1]) / a.dq1;
-        const double curl3 = (E2[t] - E2[m1]) / a.dq1 - (E1[t] - E1[m2]) / a.dq2;
+        const int m1 = g2 * a.Nq1g + down(g1, a.Nq1g);     // shift(.., 1, 0)
+        const int m2 = down(g2, a.Nq2g) * a.Nq1g + g1;     // shift(.., 0, 1)
+        const double curl1 = field_div(E3[t] - E3[m2], a.dq2, r2);
+        const double curl2 = field_div(-(E3[t] - E3[m1]), a.dq1, r1);
+        const double curl3 = field_div(E2[t] - E2[m1], a.dq1, r1) -
+                             field_div(E1[t] - E1[m2], a.dq2, r2);
         a.yee[3 * n + t] = a.yee[3 * n + t] + -a.dt * curl1;
         a.yee[4 * n + t] = a.yee[4 * n + t] + -a.dt * curl2;
         a.yee[5 * n + t] = a.yee[5 * n + t] + -a.dt * curl3;
@@ -117,9 +134,9 @@ __device__ __forceinline__ void fdtd_to_cell(const FieldArgs& a, int first, int 
     const double* y = a.yee;
     for (int t = first; t < n; t += step) {
         const int g1 = t % a.Nq1g, g2 = t / a.Nq1g;
-        const int p1 = g2 * a.Nq1g + wrapi(g1 + 1, a.Nq1g);
-        const int p2 = wrapi(g2 + 1, a.Nq2g) * a.Nq1g + g1;
-        const int p12 = wrapi(g2 + 1, a.Nq2g) * a.Nq1g + wrapi(g1 + 1, a.Nq1g);
+        const int p1 = g2 * a.Nq1g + up(g1, a.Nq1g);
+        const int p2 = up(g2, a.Nq2g) * a.Nq1g + g1;
+        const int p12 = up(g2, a.Nq2g) * a.Nq1g + up(g1, a.Nq1g);
         const double e1 = 0.5 * (y[0 * n + t] + y[0 * n + p1]);
         const double e2 = 0.5 * (y[1 * n + t] + y[1 * n + p2]);
         const double e3 = y[2 * n + t];
@@ -151,7 +168,8 @@ __global__ void fdtd_to_cell_kernel(FieldArgs a) {
 // The whole update as one cluster of CTAs: the same passes in the same order,
 // the cluster barrier (release / acquire) between them instead of a launch each.
 // What bounds it: the latency of the passes.  64^2 cells: six launches were 36 us
-// of a 312 us step (FP32, 64^2 x 32^2), 301 us with this one.
+// of a 312 us step (FP32, 64^2 x 32^2), 301 us with this one; the kernel itself
+// 26 us with IEEE divisions and index remainders, 20 us with reciprocals.
 __global__ void __cluster_dims__(kFieldCluster, 1, 1) __launch_bounds__(kFieldThreads)
 fdtd_step_kernel(FieldArgs a) {
     const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;

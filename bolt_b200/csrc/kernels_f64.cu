@@ -22,7 +22,10 @@ cudaError_t launch_field_halo(const FieldArgs& a, cudaStream_t st) {
 
 cudaError_t launch_fdtd(const FieldArgs& a, cudaStream_t st, long long* launches) {
     if (a.Nq1g * a.Nq2g <= kFieldClusterCells) {
-        fdtd_step_kernel<<<kFieldCluster, kFieldThreads, 0, st>>>(a);
+        // the cells spread over all CTAs of the cluster: one per thread while they last
+        const int per = (a.Nq1g * a.Nq2g + kFieldCluster - 1) / kFieldCluster;
+        const int threads = per < kFieldThreads ? (per + 31) / 32 * 32 : kFieldThreads;
+        fdtd_step_kernel<<<kFieldCluster, threads, 0, st>>>(a);
         if (launches) *launches += 1;
         return cudaGetLastError();
     }
