@@ -347,6 +347,7 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
                       (((size_t)ctx->Np * ctx->elem) % 16 == 0) && get_encode_fn() != nullptr;
     if (p.fields_enabled)
         ctx->pshape = choose_pshape(g.N_p1, g.N_p2, g.N_p3, ctx->elem,
+                                    ctx->elem == 4 && p.recon_p != BOLT_RECON_WENO5,
                                     (long long)g.N_q1 * g.N_q2 * g.N_s, current_sm_count());
     ctx->at_n = 1;
     ctx->pair_enabled = getenv("BOLT_NO_PAIR") == nullptr;

@@ -505,33 +505,6 @@ struct ConstPairWalkerT {
     }
 };
 
-// Face walker of one p-line: the reference-order faces in FP64, the sliding
-// third-difference form (which returns twice the face value) in FP32
-template <int RECON, bool EXACT, typename T> struct PLineWalker {
-    typedef Weno5Side<T> Side;
-    FaceWalker<RECON, EXACT, T> w;
-    __device__ __forceinline__ T first(T y0, T y1, T y2, T y3, T y4, bool right, const Side& S) {
-        return w.first(y0, y1, y2, y3, y4, right, S);
-    }
-    __device__ __forceinline__ T next(T y0, T y1, T y2, T y3, T y4, bool right, const Side& S) {
-        return w.next(y0, y1, y2, y3, y4, right, S);
-    }
-    __device__ __forceinline__ static T flux(T C, T face) { return C * face; }
-};
-template <> struct PLineWalker<BOLT_RECON_WENO5, false, float> {
-    typedef Weno5PairT<float, float> Side;
-    Weno5PairWalkerT<float, float> w;
-    __device__ __forceinline__ float first(float y0, float y1, float y2, float y3, float y4, bool,
-                                           const Side& S) {
-        return w.first(y0, y1, y2, y3, y4, S);
-    }
-    __device__ __forceinline__ float next(float y0, float y1, float y2, float y3, float y4, bool,
-                                          const Side& S) {
-        return w.next(y0, y1, y2, y3, y4, S);
-    }
-    __device__ __forceinline__ static float flux(float C, float face) { return (0.5f * C) * face; }
-};
-
 // ---------------------------------------------------------------------------
 // Per-thread asynchronous global -> shared copies (cp.async, 4 bytes, cached
 // in L1), committed in groups; wait_group<N> returns once at most N of this

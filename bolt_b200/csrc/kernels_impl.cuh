@@ -82,6 +82,11 @@ static cudaError_t plaunch(const PStageArgs& a, dim3 grid, int threads, size_t s
     auto k = pstage_kernel<BOLT_T, BOLT_EXACT, RECON>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
+    // all of the SM's shared memory: it holds the blocks of more CTAs than the
+    // default split of it with L1 does (12 of 64^2 x 32^2 FP32)
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     k<<<grid, threads, smem, st>>>(a);
     return cudaGetLastError();

@@ -110,13 +110,16 @@ struct PShape {
 };
 
 // A thread's work on one axis is rounds x (piece + 3): a piece costs its cells
-// and about three more for the walker's start.  The shape minimises thread-time
+// and about three more for the walker's start; `pairs`: a thread walks two pieces
+// side by side (seg counts the pairs).  The shape minimises thread-time
 // of a CTA, scaled up while the SM holds fewer than 24 warps of this launch
 // (latency not hidden): 2D blocks take the fewest threads that still fill the
 // SM, small q-grids take as many threads as shorten the walk.
-inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, long long ctas, int sms) {
+inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, bool pairs, long long ctas,
+                            int sms) {
     const int n[3] = {n1, n2, n3};
     const int Np = n1 * n2 * n3;
+    const int lanes = pairs ? 2 : 1;
     PShape best;
     best.smem = 2 * (size_t)pstage_pitch(n1) * n2 * n3 * elem + (size_t)(n1 + n2 + n3) * 8;
     best.threads = 32;
@@ -135,7 +138,8 @@ inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, long long ctas,
             if (n[ax] == 1) continue;
             double c_best = 1e300;
             for (int s = 1; s <= n[ax]; ++s) {
-                const int len = (n[ax] + s - 1) / s;
+                const int len = (n[ax] + lanes * s - 1) / (lanes * s);
+                if (s > 1 && lanes * (s - 1) * len >= n[ax]) continue;
                 const double c = (double)(((long long)Np / n[ax] * s + t - 1) / t) * (len + 3.0);
                 if (c < c_best - 1e-9) {
                     c_best = c;

@@ -17,12 +17,20 @@
 // neighbouring lines: axis 1 reads at the odd pitch and axes 2, 3 read
 // consecutive p1, both without bank conflicts.
 //
-// What bounds it: instruction issue (shared-memory loads and the face
-// arithmetic), not memory.  On 64^2 x 32^2
-// cells a stage takes 42 us in FP32 (88 us with every face worked out from
-// scratch by one thread per cell); a minmod RK2 step of 32^2 x 20^3 cells
-// went from 967 to 419 us.
+// What bounds it: instruction issue (shared-memory loads, indices and the face
+// arithmetic), not memory.  64^2 x 32^2 cells, WENO5: a stage took 88 us in FP32 and
+// 150 us in FP64 with every face worked out from scratch by one thread per cell,
+// here 41 us and 85 us.  A minmod RK2 step of 32^2 x 20^3 FP32 cells went from
+// 967 us to 283 us.
+//
+// FP32 threads walk two pieces of a line side by side as an f32x2 pair, except
+// for WENO5: its walkers carry enough state that the pair's second set of
+// pointers and the longer pieces cost more than the paired arithmetic saves (41 us
+// a stage by single pieces, 44 us by pairs; minmod 105 us by single pieces, 94 us
+// by pairs).
 #pragma once
+
+#include <type_traits>
 
 #include "fvm_kernels.cuh"
 
@@ -176,8 +184,55 @@ __device__ __forceinline__ bool pstage_combine(const PStageArgs& a, const T* fb,
     return bad;
 }
 
+// Lane value and face walker of a p-line: FP64 walks one piece per thread with
+// the reference-order faces, FP32 one (WENO5) or an f32x2 pair of pieces of the
+// same line with the walkers of the paired q-stage kernel (twice the face value).
+template <int RECON, typename T> struct PWalk;
+template <int RECON> struct PWalk<RECON, double> {
+    typedef double P;
+    typedef Weno5Side<double> Side;
+    FaceWalker<RECON, true, double> w;
+    __device__ __forceinline__ P first(const P (&y)[5], bool right, const Side& S) {
+        return w.first(y[0], y[1], y[2], y[3], y[4], right, S);
+    }
+    __device__ __forceinline__ P next(P y0, P y1, P y2, P y3, P y4, bool right, const Side& S) {
+        return w.next(y0, y1, y2, y3, y4, right, S);
+    }
+    __device__ __forceinline__ static double scale(double C) { return C; }
+};
+template <int RECON> struct PWalk<RECON, float> {
+    static constexpr bool WENO = RECON == BOLT_RECON_WENO5;
+    typedef typename std::conditional<WENO, float, float2>::type P;
+    typedef Weno5PairT<float, P> Side;
+    typename std::conditional<
+        RECON == BOLT_RECON_MINMOD, MinmodPairWalkerT<float>,
+        typename std::conditional<
+            RECON == BOLT_RECON_PPM, PpmPairWalkerT<float>,
+            typename std::conditional<RECON == BOLT_RECON_PC, ConstPairWalkerT<float>,
+                                      Weno5PairWalkerT<float, P>>::type>::type>::type w;
+    __device__ __forceinline__ P first(const P (&y)[5], bool, const Side& S) {
+        return w.first(y[0], y[1], y[2], y[3], y[4], S);
+    }
+    __device__ __forceinline__ P next(P y0, P y1, P y2, P y3, P y4, bool, const Side& S) {
+        return w.next(y0, y1, y2, y3, y4, S);
+    }
+    __device__ __forceinline__ static float scale(float C) { return 0.5f * C; }
+};
+
+// the next value of a circular line of n elements: m the index of *p
+template <typename T>
+__device__ __forceinline__ T line_next(const T*& p, int& m, int n, int stride) {
+    const T v = *p;
+    p += stride;
+    if (++m == n) {
+        m = 0;
+        p -= n * stride;
+    }
+    return v;
+}
+
 template <typename T, bool EXACT, int RECON>
-__global__ void __launch_bounds__(PTHREADS_MAX)
+__global__ void __launch_bounds__(PTHREADS_MAX, sizeof(T) == 4 ? 2 : 1)
 pstage_kernel(const __grid_constant__ PStageArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int n1 = a.Np1, n2 = a.Np2, n3 = a.Np3;
@@ -243,19 +298,24 @@ pstage_kernel(const __grid_constant__ PStageArgs a) {
     }
 
     // a single-cell axis contributes exactly zero; `term` keeps one axis alone
+    typedef PWalk<RECON, T> Walk;
+    typedef typename Walk::P P;
+    constexpr int LN = LaneOf<P>::n;         // pieces a thread walks side by side
     bool first = true;
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
         const int n = ax == 0 ? n1 : (ax == 1 ? n2 : n3);
         if (n == 1 || (a.term && a.term != ax + 1)) continue;
-        const int lines = a.Np / n, items = lines * a.seg[ax];
-        const int len = (n + a.seg[ax] - 1) / a.seg[ax];
+        const int lines = a.Np / n, seg = a.seg[ax], items = lines * seg;
+        const int len = (n + LN * seg - 1) / (LN * seg);
         const int stride = ax == 0 ? 1 : (ax == 1 ? pitch : n2 * pitch);
         const T inv = T(1.0 / (ax == 0 ? a.sg.dp1[s] : (ax == 1 ? a.sg.dp2[s] : a.sg.dp3[s])));
         const PDiv DL(lines);
         for (int it = tid; it < items; it += nt) {
+            // pieces sg and sg + seg of the line
             int line, base;
-            const int b = DL.div(it, &line) * len, e = min(n, b + len);
+            const int sg = DL.div(it, &line);
+            const int b = sg * len, e = min(n, b + len);
             if (b >= e) continue;
             // the line's first element and its acceleration
             double Cd;
@@ -274,30 +334,65 @@ pstage_kernel(const __grid_constant__ PStageArgs a) {
             const T C = T(Cd);
             const bool right = C > T(0);
             // window of the left face of cell i: cells i - 3 .. i + 1 (upwind from
-            // the left), or i - 2 .. i + 2, circular; m is the next one to load
-            int m = b + (right ? -3 : -2);
-            while (m < 0) m += n;
-            const T* __restrict__ fl = fb + base;
+            // the left), or i - 2 .. i + 2, circular
+            const T* p[LN];
+            int m[LN], cell[LN];
+#pragma unroll
+            for (int h = 0; h < LN; ++h) {
+                cell[h] = b + h * seg * len;
+                m[h] = cell[h] + (right ? -3 : -2);
+                while (m[h] < 0) m[h] += n;
+                while (m[h] >= n) m[h] -= n;          // an empty second piece
+                p[h] = fb + base + m[h] * stride;
+            }
             auto take = [&]() {
-                const T v = fl[m * stride];
-                if (++m == n) m = 0;
+                P v;
+#pragma unroll
+                for (int h = 0; h < LN; ++h) comp(v, h) = line_next(p[h], m[h], n, stride);
                 return v;
             };
-            typedef PLineWalker<RECON, EXACT, T> Walker;
-            typename Walker::Side S;
+            typename Walk::Side S;
             S.set(right);
-            Walker W;
-            T y0 = take(), y1 = take(), y2 = take(), y3 = take(), y4 = take();
-            T Fprev = Walker::flux(C, W.first(y0, y1, y2, y3, y4, right, S));
-            T* __restrict__ al = acc + base + b * stride;
-#pragma unroll 4
-            for (int i = b; i < e; ++i, al += stride) {
-                y0 = y1; y1 = y2; y2 = y3; y3 = y4;
-                y4 = take();
-                const T Fn = Walker::flux(C, W.next(y0, y1, y2, y3, y4, right, S));
-                const T d = (Fn - Fprev) * inv;
-                *al = first ? d : *al + d;
-                Fprev = Fn;
+            Walk W;
+            P y[5];
+#pragma unroll
+            for (int t = 0; t < 5; ++t) y[t] = take();
+            const P vC = LaneOf<P>::splat(Walk::scale(C));
+            P Fprev = mul2(vC, W.first(y, right, S));
+            T* al = acc + base + b * stride;
+            const int other = seg * len * stride;     // from one piece's cell to the other's
+            int left = e - b, left2 = n - cell[LN - 1];
+            // pairs: five faces per round, the window rotates through its registers
+            // (32^2 x 20^3 minmod: 281 us per RK2 step against 284 us unrolled by 4)
+            constexpr int U = LN == 1 ? 1 : 5, ROUNDS = LN == 1 ? 4 : 1;
+#pragma unroll ROUNDS
+            while (left > 0) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (left <= 0) break;
+                    const P v = take();
+                    P Fn;
+                    if constexpr (U == 1) {
+                        y[0] = y[1]; y[1] = y[2]; y[2] = y[3]; y[3] = y[4]; y[4] = v;
+                        Fn = W.next(y[0], y[1], y[2], y[3], y[4], right, S);
+                    } else {
+                        y[u] = v;
+                        Fn = W.next(y[(u + 1) % 5], y[(u + 2) % 5], y[(u + 3) % 5],
+                                    y[(u + 4) % 5], y[u], right, S);
+                    }
+                    Fn = mul2(vC, Fn);
+                    P d = mul2(sub2(Fn, Fprev), LaneOf<P>::splat(inv));
+                    Fprev = Fn;
+#pragma unroll
+                    for (int h = 0; h < LN; ++h) {
+                        if (h && left2 <= 0) break;
+                        T* q = al + h * other;
+                        *q = first ? comp(d, h) : *q + comp(d, h);
+                    }
+                    al += stride;
+                    --left;
+                    --left2;
+                }
             }
         }
         first = false;
