@@ -82,7 +82,9 @@ __host__ __device__ inline PLayout qpair_layout(int ntab, int bgk, unsigned elem
     L.x = o;  o += 2 * kPairHaloElems * elem;     // double-buffered halo tile
     o = qalign(o, 1024);
     L.o1 = o; o += tile;                          // out1 staging (128B swizzle)
-    L.o2 = o; o += tile;                          // out2 staging
+    // out2 staging (FP32 on any grid stores out2 from registers: without this
+    // tile, and the tables of N_p1 + N_p2 + N_p3 up to 90, two CTAs share an SM)
+    L.o2 = o; o += any && elem == 4 ? 0u : tile;
     L.b1 = o; o += 2 * tile;                      // base1 tile, double-buffered
     L.d1 = o; o += tile;                          // q1 part of df/dt (prologue: Maxwellian
                                                   // parameters of the 64 q-cells)

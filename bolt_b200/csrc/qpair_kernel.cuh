@@ -48,8 +48,8 @@
 // goes from the q2 walkers' registers to memory.  The scalar kernel (8 warps,
 // four divisions a face, single-buffered halo) left the FP64 pipe idle most of
 // the time: an RK4 step of 64^2 x 24^3 cells took 9.62 ms, here 3.59 ms (its
-// bytes alone 1.2 ms; 3.78 ms with the q1 walk rolled); what bounds it now is the latency of the dependent FP64
-// chains at 16 warps per SM.
+// bytes alone 1.2 ms; 3.78 ms with the q1 walk rolled); what bounds it now is the
+// latency of the dependent FP64 chains at 16 warps per SM.
 //
 // QG_ANY, QG_CURRENTS: any grid.  The halo and base tiles come by TMA where rows
 // are multiples of 16 bytes (cells outside the array read as zero), else by
@@ -57,8 +57,11 @@
 // outputs go from the q2 walkers' registers to memory under a mask, and the
 // accumulator's increment by one red.global.add per element.  An RK2 step of
 // 75 x 50 x 45 x 35 FP32 cells between mirrors (rows of 6300 bytes, by copies)
-// took 551 us on the scalar kernel, here 186 us; a currents stage of 64^2 x 32^2
-// FP32 cells went from 78 to about 35 us.
+// took 551 us on the scalar kernel, here 150 us (180 us while an out2 tile that
+// FP32 does not need there left room for one CTA per SM).  The currents add up
+// eight cells at a time over the warp: a currents stage of 64^2 x 32^2 FP32 cells
+// went from 78 us to 37 us, and with nine exchanges instead of forty to 29 us
+// (FP64: from 106 us to 82 us).
 //
 // Launch conditions (checked by the host): FP32 or FP64, any reconstruction in q, 8x8 tiling,
 // N_q1, N_q2 multiples of 8 and at least 2 N_g, N_p multiple of 32, N_p1
@@ -337,6 +340,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     constexpr bool BX = MODE == QP_X1 || MODE == QP_X2 || MODE == QP_K;   // no base tiles
     constexpr bool KOUT = MODE == QP_K;
     constexpr bool ANY = GEN != QG_TILES, JCUR = GEN == QG_CURRENTS;
+    constexpr int JN = JCUR ? 8 : 1;
     static_assert(!JCUR || KOUT, "currents: the stages whose q-part is written alone");
     static_assert(!EXACT || F64, "the reference's operation order: FP64");
     constexpr bool HAS2 = MODE == QP_X2 || MODE == QP_B1R2;
@@ -488,9 +492,10 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     double* jacc = reinterpret_cast<double*>(sm + Lo.jacc);
     if (JCUR)
         for (int c = tid; c < NQ * 3; c += NT) jacc[c] = 0.0;
-    auto add_current = [&](int cell, int comp, double v) {
-        v = warp_sum(v);
-        if (lane == 0) jacc[cell * 3 + comp] += v;
+    // (eight cells at a time, cell0 + k * step, by warp_sum8)
+    auto add_currents = [&](double (&v)[TQ], int cell0, int step, int comp) {
+        const double sum = warp_sum8(v);
+        if ((lane & 3) == 0) jacc[(cell0 + (lane >> 2) * step) * 3 + comp] += sum;
     };
     // any N_p1: velocities of the chunk's 32 p for phase C, by chunk parity
     double* vtab = reinterpret_cast<double*>(sm + Lo.vtab);
@@ -583,6 +588,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                 double fp = WX.first(y0, y1, y2, y3, y4, right, SX);
                 double Fp = v1 * fp;
                 double* db = o2s + lp * TQ * PW + lane;
+                double jl[TQ];
 #pragma unroll
                 for (int c = 0; c < TQ; ++c) {
                     y0 = y1; y1 = y2; y2 = y3; y3 = y4;
@@ -595,33 +601,29 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                         const double f0 = (t1[c * TW] * t2[c * TW]) * t3[c * TW];
                         db[c * PW] = div_by(-(fcell - f0), tau, inv_tau);
                     }
-                    if (JCUR) {
-                        add_current(lp * TQ + c, 0, pvalid ? fp * V1 : 0.0);
-                        add_current(lp * TQ + c, 2, pvalid ? fcell * V3 : 0.0);
-                    }
+                    if (JCUR) jl[c] = pvalid ? fp * V1 : 0.0;
                     Fp = Fn;
                     fp = fn;
+                }
+                if (JCUR) {
+                    add_currents(jl, lp * TQ, 1, 0);
+                    const double* cells = Xb + ((lp + HALO) * HX + HALO) * PW + lane;
+#pragma unroll
+                    for (int c = 0; c < TQ; ++c) jl[c] = pvalid ? cells[c * PW] * V3 : 0.0;
+                    add_currents(jl, lp * TQ, 1, 2);
                 }
             } else {
             Walker W;
             const P vq = LaneOf<P>::splat(E(0.5) * v1 * inv_dq1);   // walker: 2x face value
             P Fprev = W.first(y0, y1, y2, y3, y4, S);
+            P jf[JN];                                  // left faces of the cells (currents)
 #pragma unroll
             for (int c = 0; c < TQ; ++c) {
                 y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                 y4 = ld(ra + (c + 5) * PW, rb);
                 const P Fn = W.next(y0, y1, y2, y3, y4, S);
                 P d = mul2(sub2(Fprev, Fn), vq);
-                if (JCUR) {
-                    P fc = right ? y2 : y1;
-#pragma unroll
-                    for (int h = 0; h < ROWS; ++h) {
-                        const int cell = (lp + h) * TQ + c;
-                        // (the walker's value is twice the face's)
-                        add_current(cell, 0, pvalid ? double(comp(Fprev, h)) * (0.5 * V1) : 0.0);
-                        add_current(cell, 2, pvalid ? double(comp(fc, h)) * V3 : 0.0);
-                    }
-                }
+                if (JCUR) jf[c % JN] = Fprev;
                 Fprev = Fn;
                 if (BGK) {
                     // the cell itself is the window's y2 (right-moving) or y1
@@ -630,6 +632,22 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                     d = fma2(sub2(f0, fcell), inv_tau, d);
                 }
                 st(da + c * PW, TQ * PW, d);
+            }
+            if (JCUR) {
+                // (the walker's value is twice the face's)
+                const double w1 = 0.5 * V1;
+                const E* cells = Xb + ((lp + HALO) * HX + HALO) * PW + lane;
+#pragma unroll
+                for (int h = 0; h < ROWS; ++h) {
+                    double jl[TQ];
+#pragma unroll
+                    for (int c = 0; c < TQ; ++c) jl[c] = pvalid ? double(comp(jf[c % JN], h)) * w1 : 0.0;
+                    add_currents(jl, (lp + h) * TQ, 1, 0);
+#pragma unroll
+                    for (int c = 0; c < TQ; ++c)
+                        jl[c] = pvalid ? double(cells[(h * HX + c) * PW]) * V3 : 0.0;
+                    add_currents(jl, (lp + h) * TQ, 1, 2);
+                }
             }
             }
             // the store of chunk k-1 must be done reading the staging tiles
@@ -655,6 +673,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                 ExactWalker WX;
                 double fp = WX.first(y0, y1, y2, y3, y4, right, SX);
                 double Fp = v2 * fp;
+                double jl[TQ];
 #pragma unroll
                 for (int r = 0; r < TQ; ++r) {
                     y0 = y1; y1 = y2; y2 = y3; y3 = y4;
@@ -662,25 +681,34 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
                     const double fn = WX.next(y0, y1, y2, y3, y4, right, SX);
                     const double Fn = v2 * fn;
                     dq[r] = div_by(Fn - Fp, a.dq2, inv_dq2);
-                    if (JCUR) add_current(r * TQ + lp, 1, pvalid ? fp * V2 : 0.0);
+                    if (JCUR) jl[r] = pvalid ? fp * V2 : 0.0;
                     Fp = Fn;
                     fp = fn;
                 }
+                if (JCUR) add_currents(jl, lp, TQ, 1);
             } else {
             Walker W;
             P Fprev = W.first(y0, y1, y2, y3, y4, S);
+            P jf[JN];                                  // bottom faces of the cells
 #pragma unroll
             for (int r = 0; r < TQ; ++r) {
                 y0 = y1; y1 = y2; y2 = y3; y3 = y4;
                 y4 = ld(ca + (r + 5) * HX * PW, cb);
                 const P Fn = W.next(y0, y1, y2, y3, y4, S);
                 dq[r] = sub2(Fprev, Fn);
-                if (JCUR)
-#pragma unroll
-                    for (int h = 0; h < ROWS; ++h)
-                        add_current(r * TQ + lp + h, 1,
-                                    pvalid ? double(comp(Fprev, h)) * (0.5 * V2) : 0.0);
+                if (JCUR) jf[r % JN] = Fprev;
                 Fprev = Fn;
+            }
+            if (JCUR) {
+                const double w2 = 0.5 * V2;
+#pragma unroll
+                for (int h = 0; h < ROWS; ++h) {
+                    double jl[TQ];
+#pragma unroll
+                    for (int r = 0; r < TQ; ++r)
+                        jl[r] = pvalid ? double(comp(jf[r % JN], h)) * w2 : 0.0;
+                    add_currents(jl, lp + h, TQ, 1);
+                }
             }
             }
             if (!BX && !failed &&
