@@ -126,6 +126,7 @@ struct BoltCtx {
     LineShape line;
     int pair_shape_ok;      // grid/method meet the paired kernel's shape conditions
     int any_shape_ok;       // ... or those of its form for any grid
+    PSplit split_k;         // p-split of the tile kernels' stages that write k alone
 };
 
 #define CK(x)                                             \
@@ -330,7 +331,8 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         // BOLT_CHUNKS_PER_SPLIT fixes the split instead (tests run one problem
         // under several splits; results differ only in the order of the FP64
         // moment partial sums)
-        if (const char* env = getenv("BOLT_CHUNKS_PER_SPLIT")) {
+        const char* env = getenv("BOLT_CHUNKS_PER_SPLIT");
+        if (env) {
             const int c = atoi(env);
             if (c >= 1) {
                 sp.chunks_per_split = c < nchunks ? c : nchunks;
@@ -339,6 +341,14 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         }
         ctx->chunks_per_split = sp.chunks_per_split;
         ctx->nsplit = sp.nsplit;
+        // the stages of a run with fields that write k alone leave no partial
+        // sums, so their split only has to fill the GPU (64^2 x 32^2 FP64: 128
+        // CTAs in one wave instead of 256 in two)
+        ctx->split_k = sp;
+        if (p.fields_enabled && (ctx->pair_shape_ok || ctx->any_shape_ok) && !env)
+            ctx->split_k = choose_psplit(nchunks, base_ctas, current_sm_count(),
+                                         qpair_smem(ctx->ntab, ctx->bgk, ctx->elem,
+                                                    !ctx->pair_shape_ok));
         if (ctx->line_ok && ctx->line.threads > sp.chunks_per_split * PW)
             ctx->line.threads = sp.chunks_per_split * PW;
     }
@@ -843,6 +853,11 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         const CUtensorMap* m = (uintptr_t)a.base1 % 16 == 0
             ? get_tmap(ctx, a.base1, TMAP_TILE) : nullptr;
         if (m) a.tm_b1 = *m; else a.use_tma = 0;
+    }
+    if ((pair || any) && write_k && !want_j) {
+        a.nsplit = ctx->split_k.nsplit;
+        a.chunks_per_split = ctx->split_k.chunks_per_split;
+        grid.y = g.N_s * ctx->split_k.nsplit;
     }
     const size_t smem = pair || any ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, any)
                                     : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk,
