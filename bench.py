@@ -526,7 +526,7 @@ def run_ours(args, rank, world, local_rank):
         fp64 = {'value': job_value(cells, world, ms64), 'ms_per_step': ms64,
                 'bytes_per_cell_update': 136,
                 'hbm_frac': 136 * cells / (ms64 * 1e-3) / (peak * 1e9),
-                'kernel': 'qstage_kernel<double> (reference operation order, -fmad=false)',
+                'kernel': 'qpair_kernel<double>, reference operation order (-fmad=false)',
                 'fp32_rel_l2_error_vs_fp64': err(mom32),
                 'fp32_over_fp64': ms64 / ms,
                 'error_after_steps': args.warmup + args.steps}
