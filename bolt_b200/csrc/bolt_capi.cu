@@ -320,7 +320,8 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         const int nchunks = (ctx->Np + PW - 1) / PW;
         const long long base_ctas = (long long)ctx->ntiles1 * ctx->ntiles2 * g.N_s;
         PSplit sp = choose_psplit(nchunks, base_ctas, current_sm_count(), smem_est);
-        ctx->line_ok = g.N_q2 == 1 && p.bc_q2 == BOLT_BC_PERIODIC && g.N_p2 == 1 && g.N_p3 == 1;
+        ctx->line_ok = g.N_q2 == 1 && p.bc_q2 == BOLT_BC_PERIODIC && g.N_p2 == 1 &&
+                       g.N_p3 == 1 && (long long)g.N_q1 * g.N_s * ctx->Np <= kLineCells;
         if (ctx->line_ok) {
             ctx->line = choose_line(g.N_q1, g.N_s, ctx->Np, current_sm_count());
             if (!p.fields_enabled) {

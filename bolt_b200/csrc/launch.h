@@ -63,6 +63,13 @@ inline PSplit choose_psplit(int nchunks, long long base_ctas, int sms, size_t sm
     return PSplit{(nchunks + best_cps - 1) / best_cps, best_cps};
 }
 
+// Cells up to which the line kernel takes a 1D1V stage; larger grids fill the
+// GPU with the scalar kernel's 64-cell tiles, which read f through shared memory.
+// RK4 step of 300 x 900 cells: 84 us here, 119 us by tiles (FP32 minmod; FP64 91
+// and 134 us); of 500 x 1000: 144 and 134 us (FP64 174 and 161 us, FP32 WENO5 148
+// and 141 us).
+constexpr long long kLineCells = 3 << 17;
+
 // Launch shape of the 1D1V q-stage (line_kernel): q-cells per thread, p-threads
 // per CTA, p-chunks of 32 per CTA.  R grows while the threads still fill about
 // two warps per scheduler; the p-range of a q-cell is split over CTAs only while
