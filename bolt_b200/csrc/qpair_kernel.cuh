@@ -447,6 +447,11 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
         load_b(k_begin, 0);
         load_b(k_begin + 1, 1);
     }
+    // the currents' sums: zeroed by whichever thread, added to by the warp whose
+    // cells they are, so the prologue's barriers have to stand in between
+    double* jacc = reinterpret_cast<double*>(sm + Lo.jacc);
+    if (JCUR)
+        for (int c = tid; c < NQ * 3; c += NT) jacc[c] = 0.0;
     // p3 rows of this CTA's p-range (the tables hold only those)
     const int p3lo = (k_begin * PW) / (Np1 * Np2);
     const int p_last = ANY ? min(k_end * PW, Np) - 1 : k_end * PW - 1;
@@ -486,12 +491,9 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
     // columns 2(w-4), 2(w-4)+1; single rows: q1 walkers (warps 0-7) row w, q2
     // walkers (warps 8-15) column w-8; each walks the 8 cells of its line
     const bool q1w = warp < NWARP / 2;
-    // currents of the chunks so far, [q-cell][3]: a warp's sum over the 32 p of
+    // currents of the chunks so far, jacc[q-cell][3]: a warp's sum over the 32 p of
     // each chunk, added chunk by chunk (face value * v1 at left faces and f * v3
     // by the q1 walkers, face value * v2 at bottom faces by the q2 walkers)
-    double* jacc = reinterpret_cast<double*>(sm + Lo.jacc);
-    if (JCUR)
-        for (int c = tid; c < NQ * 3; c += NT) jacc[c] = 0.0;
     // (eight cells at a time, cell0 + k * step, by warp_sum8)
     auto add_currents = [&](double (&v)[TQ], int cell0, int step, int comp) {
         const double sum = warp_sum8(v);

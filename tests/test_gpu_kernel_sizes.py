@@ -98,6 +98,28 @@ def test_tile_kernels_write_the_scalar_kernels_bits(monkeypatch, q, p, source):
         assert np.array_equal(out[0], out[1])
 
 
+@pytest.mark.parametrize('q,p', [((9, 8), (33, 3, 1)), ((16, 16), (8, 4, 2))])
+@pytest.mark.parametrize('chunks', [None, '1'])
+def test_currents_write_the_scalar_kernels_bits(monkeypatch, q, p, chunks):
+    """FP64 currents by the tile kernel and by the scalar kernel, split the same
+    way: the fields they drive have the same bits, also where a CTA's first chunk
+    of p is its only one, in every run."""
+    if chunks:
+        monkeypatch.setenv('BOLT_CHUNKS_PER_SPLIT', chunks)
+    spec = _spec(q, p, fields_enabled=True, source_enabled=False, integrator='RK4')
+
+    def fields():
+        nls = make_solver(spec, 'fp64')
+        nls.strang_timestep(5e-4)
+        return nls.fields_solver.yee_grid_EM_fields.cpu().numpy()
+    tiles = [fields() for _ in range(8)]
+    monkeypatch.setenv('BOLT_NO_PAIR', '1')
+    scalar = fields()
+    assert np.abs(scalar).max() > 0
+    for t in tiles:
+        assert np.array_equal(t, scalar)
+
+
 # p-blocks: one-cell axes, two cells (the window wraps onto itself), rows of one
 # vector and off it, more lines than threads
 PBLOCKS = [(8, 1, 1), (2, 3, 1), (1, 5, 4), (5, 2, 3), (4, 4, 4), (33, 7, 1), (12, 11, 10)]
