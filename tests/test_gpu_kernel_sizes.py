@@ -186,10 +186,10 @@ def test_semi_lagrangian_source_blocks(p, precision):
     assert rel(interior(to_layout(nls.f, spec), g), interior(o.f, g)) < TOL[precision]
 
 
-@pytest.mark.parametrize('n', [(64, 64), (250, 251)])
+@pytest.mark.parametrize('n', [(64, 64), (122, 122), (123, 122), (250, 251)])
 def test_field_update_by_cluster_or_by_passes(n):
-    """One update with given currents on a grid below and one above the size at
-    which the passes become launches."""
+    """One update with given currents on grids below, at and above the size
+    (2^14 cells with the ghosts) at which the passes become launches."""
     spec = _spec(n, (2, 2, 1), fields_enabled=True, source_enabled=False)
     nls = make_solver(spec, 'fp64')
     o = Oracle(spec, to_layout(nls.f, spec))
