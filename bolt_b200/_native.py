@@ -135,6 +135,7 @@ SIGNATURES = {
     'bolt_strerror': (ctypes.c_char_p, [ctypes.c_int]),
     'bolt_launch_count': (ctypes.c_longlong, [_VP]),
     'bolt_paired_launch_count': (ctypes.c_longlong, [_VP]),
+    'bolt_line_cells': (ctypes.c_int, [_VP]),
     'bolt_split_info': (ctypes.c_int, [_VP, ctypes.POINTER(ctypes.c_int),
                                        ctypes.POINTER(ctypes.c_int)]),
     'bolt_scratch_bytes': (ctypes.c_size_t, [_VP]),

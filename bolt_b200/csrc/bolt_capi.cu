@@ -298,14 +298,12 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
                          g.N_q1 % 8 == 0 && g.N_q2 % 8 == 0 && ctx->Np % PW == 0 &&
                          g.N_p1 % 8 == 0 && 2 * g.N_ghost <= g.N_q1 &&
                          2 * g.N_ghost <= g.N_q2 && ctx->fcount < (1ull << 31);
-    if (ctx->pair_shape_ok || ctx->any_shape_ok) {
-        // their shared memory (exp tables grow with N_p1 + N_p2 + N_p3) must fit a CTA
-        int dev = 0, optin = 232448;
-        if (cudaGetDevice(&dev) == cudaSuccess)
-            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        if (qpair_smem(ctx->ntab, ctx->bgk, ctx->elem) > (size_t)optin) ctx->pair_shape_ok = 0;
-        if (qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, 1) > (size_t)optin) ctx->any_shape_ok = 0;
-    }
+    // their shared memory (exp tables grow with N_p1 + N_p2 + N_p3) must fit a CTA
+    int dev = 0, optin = 232448;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (qpair_smem(ctx->ntab, ctx->bgk, ctx->elem) > (size_t)optin) ctx->pair_shape_ok = 0;
+    if (qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, 1) > (size_t)optin) ctx->any_shape_ok = 0;
     // p-splits: the grid is (q-tiles, species x splits)
     {
         // (with fields no q-stage writes moments, and the currents' partial sums
@@ -314,14 +312,20 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         const bool tiled = p.fields_enabled
             ? ctx->pair_shape_ok && p.dtype != BOLT_F64
             : ctx->pair_shape_ok || ctx->any_shape_ok;
+        const size_t scalar_smem = qstage_smem(ctx->tiling, ctx->elem, ctx->bgk,
+                                               ctx->bgk_direct, ctx->ntab);
         const size_t smem_est = tiled
             ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, !ctx->pair_shape_ok)
-            : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk, ctx->bgk_direct, ctx->ntab);
+            : scalar_smem;
         const int nchunks = (ctx->Np + PW - 1) / PW;
         const long long base_ctas = (long long)ctx->ntiles1 * ctx->ntiles2 * g.N_s;
         PSplit sp = choose_psplit(nchunks, base_ctas, current_sm_count(), smem_est);
+        // (also where the scalar kernel's table of p-cell centres, as long as a
+        // row of f, does not fit a CTA)
         ctx->line_ok = g.N_q2 == 1 && p.bc_q2 == BOLT_BC_PERIODIC && g.N_p2 == 1 &&
-                       g.N_p3 == 1 && (long long)g.N_q1 * g.N_s * ctx->Np <= kLineCells;
+                       g.N_p3 == 1 &&
+                       (line_fits(g.N_q1, g.N_s, ctx->Np, current_sm_count()) ||
+                        scalar_smem > (size_t)optin);
         if (ctx->line_ok) {
             ctx->line = choose_line(g.N_q1, g.N_s, ctx->Np, current_sm_count());
             if (!p.fields_enabled) {
@@ -533,6 +537,7 @@ int bolt_split_info(BoltCtx* ctx, int* nsplit, int* chunks_per_split) {
     *chunks_per_split = ctx->chunks_per_split;
     return BOLT_OK;
 }
+int bolt_line_cells(BoltCtx* ctx) { return ctx && ctx->line_ok ? ctx->line.r : 0; }
 size_t bolt_scratch_bytes(BoltCtx* ctx) { return ctx ? ctx->scratch_bytes : 0; }
 
 int bolt_divergence_flag(BoltCtx* ctx) {

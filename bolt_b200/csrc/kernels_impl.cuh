@@ -52,8 +52,7 @@ static void (*pick_line(int r))(QStageArgs) {
     switch (r) {
         case 1: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 1>;
         case 2: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 2>;
-        case 4: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 4>;
-        default: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 8>;
+        default: return line_kernel<BOLT_T, BOLT_EXACT, RECON, BGK, 4>;
     }
 }
 

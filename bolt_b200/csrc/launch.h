@@ -63,13 +63,6 @@ inline PSplit choose_psplit(int nchunks, long long base_ctas, int sms, size_t sm
     return PSplit{(nchunks + best_cps - 1) / best_cps, best_cps};
 }
 
-// Cells up to which the line kernel takes a 1D1V stage; larger grids fill the
-// GPU with the scalar kernel's 64-cell tiles, which read f through shared memory.
-// RK4 step of 300 x 900 cells: 84 us here, 119 us by tiles (FP32 minmod; FP64 91
-// and 134 us); of 500 x 1000: 144 and 134 us (FP64 174 and 161 us, FP32 WENO5 148
-// and 141 us).
-constexpr long long kLineCells = 3 << 17;
-
 // Launch shape of the 1D1V q-stage (line_kernel): q-cells per thread, p-threads
 // per CTA, p-chunks of 32 per CTA.  R grows while the threads still fill about
 // two warps per scheduler; the p-range of a q-cell is split over CTAs only while
@@ -79,11 +72,25 @@ struct LineShape {
     int r, threads, chunks_per_split;
 };
 
+constexpr int kLineMaxR = 4;
+
+// Whether the line kernel takes a 1D1V stage: while four q-cells per thread are
+// enough, its lanes without a p (N_p rounded up to chunks) counted in.  Larger
+// grids fill the GPU with the scalar kernel's 64-cell tiles, which read f through
+// shared memory; eight cells per thread spill.  RK2 step with the source, line
+// kernel and tiles: 1953 x 128 cells 35 and 43 us (FP64), 1132 x 256 41 and 47 us;
+// with eight cells per thread 2421 x 128 76 and 49 us, 1367 x 256 83 and 53 us (FP32
+// 55 and 37 us).
+inline bool line_fits(int Nq1, int Ns, int Np, int sms) {
+    const long long lanes = (long long)Nq1 * Ns * ((Np + PW - 1) / PW * PW);
+    return lanes < (long long)sms * 256 * 2 * kLineMaxR;
+}
+
 inline LineShape choose_line(int Nq1, int Ns, int Np, int sms) {
     LineShape L;
     const long long cells = (long long)Nq1 * Ns * Np;
     L.r = 1;
-    while (L.r < 8 && cells / (2 * L.r) >= (long long)sms * 256) L.r *= 2;
+    while (L.r < kLineMaxR && cells / (2 * L.r) >= (long long)sms * 256) L.r *= 2;
     L.threads = Np >= LINE_THREADS ? LINE_THREADS : (Np + 31) / 32 * 32;
     const int chunks = (Np + PW - 1) / PW, per_cta = L.threads / PW;
     const long long ctas = (long long)((Nq1 + L.r - 1) / L.r) * Ns;

@@ -10,7 +10,7 @@
 // chain of latencies, so the work is cut for parallelism: a thread owns one p
 // and R consecutive q-cells, loads their R + 6 values at once and walks R + 1
 // faces in registers; nothing is staged in shared memory.  R is the largest of
-// 1, 2, 4, 8 that still fills the GPU (fewer faces computed twice).  The
+// 1, 2, 4 that still fills the GPU (fewer faces computed twice).  The
 // Maxwellian's parameters are worked out by one extra warp while the others
 // load and reconstruct.
 //

@@ -418,6 +418,10 @@ long long bolt_paired_launch_count(BoltCtx* ctx);
  * the GPU's SMs; $BOLT_CHUNKS_PER_SPLIT at context creation fixes it). */
 int  bolt_split_info(BoltCtx* ctx, int* nsplit, int* chunks_per_split);
 
+/* q-cells per thread of the 1D1V q-stage kernel, 0 where the grid's stages run
+ * another kernel. */
+int  bolt_line_cells(BoltCtx* ctx);
+
 /* Bytes of device scratch held by the context. */
 size_t bolt_scratch_bytes(BoltCtx* ctx);
 

@@ -138,27 +138,42 @@ def test_p_stage_blocks(p, precision, recon):
         < (1e-10 if precision == 'fp64' else 1e-4)
 
 
-@pytest.mark.parametrize('N', [6, 7, 64, 129])
+@pytest.mark.parametrize('N,N_p1,cells', [(6, 24, 1), (7, 24, 1), (64, 24, 1), (129, 24, 1),
+                                          (601, 130, 2), (1003, 201, 4), (2048, 24, 1),
+                                          (2049, 24, 1)])
 @pytest.mark.parametrize('precision', ['fp64', 'fp32'])
-def test_electrostatic_line(N, precision):
+def test_electrostatic_line(N, N_p1, cells, precision):
     """N_q2 = 1: E1 from the Green's function of the periodic solve, even and odd
-    lines (the Nyquist mode of an even one drops out)."""
-    spec = _spec((N, 1), (24, 1, 1), fields_enabled=True, fields_type='electrostatic',
-                 fields_solver='fft', source_enabled=False)
+    lines (the Nyquist mode of an even one drops out), up to 2,048 cells and, past
+    them, from the FFT; the q-part by the line kernel at each of its forms."""
+    spec = _spec((N, 1), (N_p1, 1, 1), fields_enabled=True, fields_type='electrostatic',
+                 fields_solver='fft', source_enabled=False, dt=5e-4 if N < 200 else 0.1 / N / 6)
     nls, o = _against_oracle(spec, precision, fields=True)
+    _line_cells(nls, cells)
     got = nls.fields_solver.cell_centered_EM_fields[:2, 0].permute(0, 2, 1).cpu().numpy()
     assert rel(got, o.fields.cell[:2]) < (1e-11 if precision == 'fp64' else 1e-5)
 
 
-# 1D1V: q-cells per thread of 1, 2, 4 and 8 (by size), partial last groups, p
-# below, at and above the CTA's threads, one and two species
-@pytest.mark.parametrize('N_q1,N_p1', [(6, 5), (9, 32), (64, 300), (601, 130), (1003, 201), (1201, 512)])
+# 1D1V: 1, 2 and 4 q-cells per thread of the line kernel (148 SMs), partial last
+# groups, p below, at and above the CTA's threads, one and two species; 0: the sizes
+# just past it and well past it, on the scalar kernel's tiles
+LINES = [(6, 5, 1), (9, 32, 1), (64, 300, 1), (601, 130, 2), (1003, 201, 4), (1183, 256, 4),
+         (1184, 256, 0), (1201, 512, 0)]
+
+
+def _line_cells(nls, cells):
+    assert nls._lib.bolt_line_cells(nls._ctx) == cells
+
+
+@pytest.mark.parametrize('N_q1,N_p1,cells', LINES)
 @pytest.mark.parametrize('precision', ['fp64', 'fp32'])
 @pytest.mark.parametrize('source', [False, True])
-def test_line(N_q1, N_p1, precision, source):
+def test_line(N_q1, N_p1, cells, precision, source):
     ns = 2 if N_q1 < 100 else 1
-    _against_oracle(_spec((N_q1, 1), (N_p1, 1, 1), source_enabled=source, mass=[1.0, 2.0][:ns],
-                          charge=[0.0] * ns, dt=0.1 / N_q1 / 6), precision)
+    nls, _ = _against_oracle(_spec((N_q1, 1), (N_p1, 1, 1), source_enabled=source,
+                                   mass=[1.0, 2.0][:ns], charge=[0.0] * ns,
+                                   dt=0.1 / N_q1 / 6), precision)
+    _line_cells(nls, cells)
 
 
 @pytest.mark.parametrize('tau', [float('inf'), 1e-2])
