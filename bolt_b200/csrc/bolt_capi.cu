@@ -320,18 +320,21 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         const int nchunks = (ctx->Np + PW - 1) / PW;
         const long long base_ctas = (long long)ctx->ntiles1 * ctx->ntiles2 * g.N_s;
         PSplit sp = choose_psplit(nchunks, base_ctas, current_sm_count(), smem_est);
-        // (also where the scalar kernel's table of p-cell centres, as long as a
-        // row of f, does not fit a CTA)
-        ctx->line_ok = g.N_q2 == 1 && p.bc_q2 == BOLT_BC_PERIODIC && g.N_p2 == 1 &&
-                       g.N_p3 == 1 &&
-                       (line_fits(g.N_q1, g.N_s, ctx->Np, current_sm_count()) ||
-                        scalar_smem > (size_t)optin);
-        if (ctx->line_ok) {
-            ctx->line = choose_line(g.N_q1, g.N_s, ctx->Np, current_sm_count());
-            if (!p.fields_enabled) {
-                sp.chunks_per_split = ctx->line.chunks_per_split;
-                sp.nsplit = (nchunks + sp.chunks_per_split - 1) / sp.chunks_per_split;
-            }
+        if (g.N_q2 == 1 && p.bc_q2 == BOLT_BC_PERIODIC && g.N_p2 == 1 && g.N_p3 == 1) {
+            const int sms = current_sm_count();
+            ctx->line = choose_line(g.N_q1, g.N_s, ctx->Np, sms);
+            const int resident = ctx->elem == 4
+                ? line_resident_f32(p.recon_q, ctx->bgk, ctx->line)
+                : line_resident_f64(p.recon_q, ctx->bgk, ctx->line);
+            // (also where the scalar kernel's table of p-cell centres, as long as
+            // a row of f, does not fit a CTA)
+            ctx->line_ok = line_fits(ctx->line, g.N_q1, g.N_s, ctx->Np, ctx->bgk, ctx->elem,
+                                     resident, sms) ||
+                           scalar_smem > (size_t)optin;
+        }
+        if (ctx->line_ok && !p.fields_enabled) {
+            sp.chunks_per_split = ctx->line.chunks_per_split;
+            sp.nsplit = (nchunks + sp.chunks_per_split - 1) / sp.chunks_per_split;
         }
         // BOLT_CHUNKS_PER_SPLIT fixes the split instead (tests run one problem
         // under several splits; results differ only in the order of the FP64

@@ -56,23 +56,36 @@ static void (*pick_line(int r))(QStageArgs) {
     }
 }
 
-template <int RECON>
-static cudaError_t lline(const QStageArgs& a, int bgk, const LineShape& shape, cudaStream_t st) {
-    void (*k)(QStageArgs) = bgk ? pick_line<RECON, true>(shape.r)
-                                : pick_line<RECON, false>(shape.r);
-    const dim3 grid((a.Nq1 + shape.r - 1) / shape.r, a.Ns * a.nsplit);
-    k<<<grid, shape.threads + (bgk ? 32 : 0), 0, st>>>(a);
-    return cudaGetLastError();
+static void (*pick_line(int recon, int bgk, int r))(QStageArgs) {
+    switch (recon) {
+        case BOLT_RECON_PC: return bgk ? pick_line<BOLT_RECON_PC, true>(r)
+                                       : pick_line<BOLT_RECON_PC, false>(r);
+        case BOLT_RECON_MINMOD: return bgk ? pick_line<BOLT_RECON_MINMOD, true>(r)
+                                           : pick_line<BOLT_RECON_MINMOD, false>(r);
+        case BOLT_RECON_PPM: return bgk ? pick_line<BOLT_RECON_PPM, true>(r)
+                                        : pick_line<BOLT_RECON_PPM, false>(r);
+        default: return bgk ? pick_line<BOLT_RECON_WENO5, true>(r)
+                            : pick_line<BOLT_RECON_WENO5, false>(r);
+    }
 }
 
 cudaError_t BOLT_CAT(launch_line_, BOLT_SUFFIX)(const QStageArgs& a, int recon, int bgk,
                                                 const LineShape& shape, cudaStream_t st) {
-    switch (recon) {
-        case BOLT_RECON_PC: return lline<BOLT_RECON_PC>(a, bgk, shape, st);
-        case BOLT_RECON_MINMOD: return lline<BOLT_RECON_MINMOD>(a, bgk, shape, st);
-        case BOLT_RECON_PPM: return lline<BOLT_RECON_PPM>(a, bgk, shape, st);
-        default: return lline<BOLT_RECON_WENO5>(a, bgk, shape, st);
+    const dim3 grid((a.Nq1 + shape.r - 1) / shape.r, a.Ns * a.nsplit);
+    pick_line(recon, bgk, shape.r)<<<grid, shape.threads + (bgk ? 32 : 0), 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+// CTAs of the line kernel that an SM holds (0: unknown)
+int BOLT_CAT(line_resident_, BOLT_SUFFIX)(int recon, int bgk, const LineShape& shape) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pick_line(recon, bgk, shape.r),
+                                                      shape.threads + (bgk ? 32 : 0), 0) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
+    return n;
 }
 
 template <int RECON>

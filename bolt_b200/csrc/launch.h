@@ -74,18 +74,6 @@ struct LineShape {
 
 constexpr int kLineMaxR = 4;
 
-// Whether the line kernel takes a 1D1V stage: while four q-cells per thread are
-// enough, its lanes without a p (N_p rounded up to chunks) counted in.  Larger
-// grids fill the GPU with the scalar kernel's 64-cell tiles, which read f through
-// shared memory; eight cells per thread spill.  RK2 step with the source, line
-// kernel and tiles: 1953 x 128 cells 35 and 43 us (FP64), 1132 x 256 41 and 47 us;
-// with eight cells per thread 2421 x 128 76 and 49 us, 1367 x 256 83 and 53 us (FP32
-// 55 and 37 us).
-inline bool line_fits(int Nq1, int Ns, int Np, int sms) {
-    const long long lanes = (long long)Nq1 * Ns * ((Np + PW - 1) / PW * PW);
-    return lanes < (long long)sms * 256 * 2 * kLineMaxR;
-}
-
 inline LineShape choose_line(int Nq1, int Ns, int Np, int sms) {
     LineShape L;
     const long long cells = (long long)Nq1 * Ns * Np;
@@ -99,6 +87,27 @@ inline LineShape choose_line(int Nq1, int Ns, int Np, int sms) {
     if (splits > most) splits = most;
     L.chunks_per_split = (int)((chunks + splits - 1) / splits);
     return L;
+}
+
+// Whether the line kernel takes a 1D1V stage.  Larger grids fill the GPU with the
+// scalar kernel's 64-cell tiles, which read f through shared memory; eight cells
+// per thread were up to 1.8 times as slow as they are.  A CTA covers a whole row of
+// p up to LINE_THREADS; there the line kernel's time goes by waves of CTAs
+// (`resident` per SM), while the tiles' hardly grows in this range.  RK2 step with the
+// source, FP32, tiles 29-33 us: one wave of four cells per thread 25 us, two 35-37 us; one
+// wave of one or two cells 16-21 us, two 25-29 us, three 35-41 us.  FP64, tiles 37-45 us: the
+// same waves 25, 37-41, 16-20, 29 and 37-41 us.  Without the source, tiles 16 us (FP64
+// 21 us): up to three waves 12-16 us, four 18-21 us.  Longer rows keep to the line
+// kernel: tiles 41-65 us, line 25-45 us.
+inline bool line_fits(const LineShape& L, int Nq1, int Ns, int Np, int bgk, size_t elem,
+                      int resident, int sms) {
+    const long long lanes = (long long)Nq1 * Ns * ((Np + PW - 1) / PW * PW);
+    if (lanes >= (long long)sms * 256 * 2 * kLineMaxR) return false;
+    if (Np > LINE_THREADS || resident < 1) return true;
+    const long long ctas = (long long)((Nq1 + L.r - 1) / L.r) * Ns;
+    const long long waves = (ctas + (long long)resident * sms - 1) / ((long long)resident * sms);
+    if (!bgk) return waves <= 3;
+    return waves <= (elem == 4 ? 2 : 3) - (L.r == 4 ? 1 : 0);
 }
 
 // SM count of the current device (148 on B200 if the query fails)
@@ -178,6 +187,7 @@ inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, bool pairs, lon
                                        dim3 grid, size_t smem, cudaStream_t st);            \
     cudaError_t launch_line_##SUFFIX(const QStageArgs& a, int recon, int bgk,               \
                                      const LineShape& shape, cudaStream_t st);              \
+    int line_resident_##SUFFIX(int recon, int bgk, const LineShape& shape);                 \
     cudaError_t launch_pstage_##SUFFIX(const PStageArgs& a, int recon, dim3 grid,           \
                                        int threads, size_t smem, cudaStream_t st);          \
     cudaError_t launch_moment_##SUFFIX(const void* f, int mid, double* out, int Ns,          \

@@ -176,6 +176,13 @@ def test_line(N_q1, N_p1, cells, precision, source):
     _line_cells(nls, cells)
 
 
+@pytest.mark.parametrize('precision,cells', [('fp64', 4), ('fp32', 0)])
+def test_line_waves(precision, cells):
+    """Two waves of CTAs of the line kernel: taken in FP64, not in FP32."""
+    nls, _ = _against_oracle(_spec((4062, 1), (64, 1, 1), dt=0.1 / 4062 / 6), precision)
+    _line_cells(nls, cells)
+
+
 @pytest.mark.parametrize('tau', [float('inf'), 1e-2])
 @pytest.mark.parametrize('q,p', [((32, 1), (40, 1, 1)), ((8, 8), (8, 4, 1)), ((9, 8), (8, 3, 1))])
 def test_infinite_collision_time(q, p, tau):
