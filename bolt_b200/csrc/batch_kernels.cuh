@@ -181,7 +181,7 @@ batch_stage_kernel(const BatchStageArgs a) {
                 const double Vh = 0.5 * V * V;
                 Weno5PairT<float, float> S;
                 S.set(right);
-                Weno5PairWalkerT<float, float> W;      // returns twice the face value
+                Weno5PairWalkerT<float, float, true> W;    // returns twice the face value
                 const float vq = 0.5f * v * inv_dq;
                 const float (*Xb)[PW] = X[b];
                 // the combine bases of this warp's 4 cells, loaded before the

@@ -412,7 +412,11 @@ __device__ __forceinline__ P second_diff(P a, P b, P c) {
 
 // Sliding walker: carries 1/beta^2 of substencils 2 and 3, the second
 // difference of substencil 3 and the third difference D3b of the last face.
-template <typename E, typename P = typename PairOf<E>::P>
+// WIDE divides the q_k by the denominator before they meet the third differences:
+// the q_k of uniform data is 1e34, so in FP32 its product with a jump beyond 3e4
+// overflows although the face value is an ordinary number.  One more operation a
+// face.
+template <typename E, typename P = typename PairOf<E>::P, bool WIDE = false>
 struct Weno5PairWalkerT {
     typedef Weno5PairT<E, P> Side;
     P q2, q3, d23, d3b;
@@ -424,9 +428,14 @@ struct Weno5PairWalkerT {
                                       const Side& S) const {
         const P ys = S.right ? y3 : y1;
         const P base = fma2(LaneOf<P>::splat(BOLT_K(E, -0.25)), d22, add2(y2, ys));
-        const P num = fma2(q3, d3b, mul2(mul2(S.r, q1), d3a));
         const P den = fma2(S.a3, q3, fma2(S.a2, q2, mul2(S.a1, q1)));
-        return fma2(num, rcp2(den), base);
+        if constexpr (WIDE) {
+            const P r = rcp2(den);
+            return fma2(mul2(q3, r), d3b, fma2(mul2(mul2(S.r, q1), r), d3a, base));
+        } else {
+            const P num = fma2(q3, d3b, mul2(mul2(S.r, q1), d3a));
+            return fma2(num, rcp2(den), base);
+        }
     }
     __device__ __forceinline__ P first(P y0, P y1, P y2, P y3, P y4, const Side& S) {
         const P d21 = second_diff(y0, y1, y2);

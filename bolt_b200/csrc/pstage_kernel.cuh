@@ -209,7 +209,7 @@ template <int RECON> struct PWalk<RECON, float> {
         typename std::conditional<
             RECON == BOLT_RECON_PPM, PpmPairWalkerT<float>,
             typename std::conditional<RECON == BOLT_RECON_PC, ConstPairWalkerT<float>,
-                                      Weno5PairWalkerT<float, P>>::type>::type>::type w;
+                                      Weno5PairWalkerT<float, P, true>>::type>::type>::type w;
     __device__ __forceinline__ P first(const P (&y)[5], bool, const Side& S) {
         return w.first(y[0], y[1], y[2], y[3], y[4], S);
     }

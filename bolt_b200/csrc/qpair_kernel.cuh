@@ -330,7 +330,7 @@ qpair_kernel(const __grid_constant__ QStageArgs a) {
         typename std::conditional<
             RECON == BOLT_RECON_PPM, PpmPairWalkerT<E, P>,
             typename std::conditional<RECON == BOLT_RECON_PC, ConstPairWalkerT<E, P>,
-                                      Weno5PairWalkerT<E, P>>::type>::type>::type;
+                                      Weno5PairWalkerT<E, P, GEN != QG_TILES>>::type>::type>::type;
     typedef Weno5PairT<E, P> Side;
     typedef FaceWalker<RECON, true, double> ExactWalker;
     typedef typename PairOf<E>::P TabP;               // table entries: row pairs
