@@ -89,7 +89,8 @@ __device__ __forceinline__ double rcp_nr(double x) {
 // a/b rounded to nearest from r = 1/b rounded to nearest: the quotient a r
 // corrected by its remainder, exact with FMA (Markstein, IBM J. Res. Dev. 34,
 // 1990).  The reference's divisions by the grid spacing and the collision time
-// share their reciprocal this way, and the WENO weights theirs.
+// share their reciprocal this way, and the WENO weights theirs.  (A quotient that
+// overflows comes out as NaN, not as infinity: a diverging run either way.)
 __device__ __forceinline__ double div_by(double a, double b, double r) {
     const double q = a * r;
     return fma(fma(-b, q, a), r, q);
@@ -190,12 +191,19 @@ template <bool EXACT, typename T> struct Weno5Walker;
 // (scaling by a power of two is exact), and the common factor 16 of the three
 // weights cancels exactly in the normalised sum.  So a face costs one
 // reciprocal for its new substencil and one for the sum, instead of four
-// divisions, and its value has the bits of the reference's expressions.  B is
-// capped where its reciprocal would leave the normal range.
+// divisions, and its value has the bits of the reference's expressions (but for
+// a reciprocal that rcp_nr rounds the other way, within 2^-80 of halfway between
+// two FP64 values).  That is for B below 2^1018; above it the reference's weights
+// turn subnormal and, from 2^1020, zero.  Here they stay normal up to 2^1022 and
+// are zero beyond, so that a face whose B all overflow is 0/0 = NaN as the
+// reference's is, and one of ordinary substencils beside an overflowing one keeps
+// to those.
 template <> struct Weno5Walker<true, double> {
     double r2, t2, r3, t3;                     // 1/B and 5/B of substencils 2 and 3
     __device__ __forceinline__ static void quotients(double beta, double& r, double& t) {
-        const double B = fmin(beta * beta, 1e300);
+        // (no infinity, whose reciprocal by Newton steps is NaN: the largest
+        // finite number's is flushed to 0)
+        const double B = fmin(beta * beta, 1.7976931348623157e308);
         r = rcp_nr(B);
         t = div_by(5.0, B, r);
     }

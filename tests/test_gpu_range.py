@@ -1,5 +1,5 @@
 """States far from the smooth, order-one ones of the other tests: jumps of large
-values beside exactly uniform data."""
+values beside exactly uniform data, and values whose squares leave the range."""
 
 import os
 import sys
@@ -97,3 +97,64 @@ def test_jump_in_a_batch(top):
         o.step(r['dt'])
     got = bs.f(0)[:, 0, :, 0].double().T.cpu().numpy()[3:-3]
     assert rel(got, o.f[3, 3:-3, 0, 0, 0, :]) < TOL['fp32']
+
+
+KERNELS = [dict(q=(32, 1), p=(40, 1, 1)),                          # line
+           dict(q=(16, 16), p=(8, 4, 1)),                          # whole tiles
+           dict(q=(9, 10), p=(9, 4, 1)),                           # any grid
+           dict(q=(9, 10), p=(9, 4, 1), scalar=True),
+           dict(q=(9, 10), p=(16, 6, 1), fields=True)]             # p-stage
+
+
+def _large_state(kernel, monkeypatch, fn):
+    if kernel.get('scalar'):
+        monkeypatch.setenv('BOLT_NO_PAIR', '1')
+    kw = dict(fields_enabled=True, fields_type='electrostatic', fields_solver='fft',
+              charge=[-1e-170]) if kernel.get('fields') else {}
+    spec = _spec(kernel['q'], kernel['p'], source_enabled=False, steps=1, **kw)
+    nls = make_solver(spec, 'fp64')
+    f0 = fn(to_layout(nls.f, spec))
+    nls.f = af_from_layout(f0).to('cuda')
+    return spec, nls, Oracle(spec, f0)
+
+
+@pytest.mark.parametrize('kernel', KERNELS)
+def test_reference_order_diverges_where_the_reference_does(monkeypatch, kernel):
+    """The smoothness indicators' squares overflow for noise of 1e90: every weight of
+    the reference is zero, its face 0/0, and the run stops."""
+    rng = np.random.default_rng(3)
+    spec, nls, o = _large_state(kernel, monkeypatch,
+                                lambda f: 1e90 * (1 + rng.random(f.shape)))
+    with np.errstate(all='ignore'), pytest.raises(SystemExit):
+        o.step(spec['dt'])
+    with pytest.raises(SystemExit):
+        for _ in range(2):                # the flag of a step is read by the next one
+            nls.strang_timestep(spec['dt'])
+            torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize('kernel', KERNELS)
+@pytest.mark.parametrize('top', [1e60, 1e90])
+def test_reference_order_beside_a_huge_value(monkeypatch, kernel, top):
+    """One value of `top`: at 1e90 the squares of its substencils overflow, faces
+    with nothing else are NaN, and the ones with an ordinary substencil keep to it."""
+    rng = np.random.default_rng(4)
+
+    def state(f):
+        f = f * (1 + 0.1 * rng.random(f.shape))
+        f[:, 3 + 4, 0, 0, 1 if f.shape[4] > 1 else 0, 5] = top
+        return f
+    spec, nls, o = _large_state(kernel, monkeypatch, state)
+    with np.errstate(all='ignore'):
+        o.fvm_step(spec['dt'])
+    nls.strang_timestep(spec['dt'])
+    g = spec['N_ghost']
+    got, want = interior(to_layout(nls.f, spec), g), interior(o.f, g)
+    assert np.array_equal(np.isfinite(got), np.isfinite(want))
+    assert np.isfinite(want).all() == (top == 1e60)
+    small = np.isfinite(want) & (np.abs(want) < 10)
+    if kernel.get('fields') and top == 1e90:
+        assert not small.any()                 # the Poisson solve spreads a NaN
+        return
+    assert small.sum() > 0.5 * want.size
+    assert rel(got[small], want[small]) < TOL['fp64']
