@@ -76,7 +76,8 @@ struct BoltCtx {
     double* momP[2];        // partial moments [nsplit][5][Ns][Nq2][Nq1]
     double* jpart;          // partial currents [nsplit][3][Ns][Nq2][Nq1]
     int cur_mom;            // index of momP holding moments of the current f
-    int cur_nsplit;         // nsplit of that buffer
+    int mom_nsplit[2];      // nsplit of the partial sums in momP[0], momP[1]
+    int q_nsplit;           // nsplit of the last q-stage launch
     const void* mom_owner;  // f pointer whose moments momP[cur_mom] holds (null: stale)
     const void* ghost_owner;
     // fields
@@ -127,6 +128,7 @@ struct BoltCtx {
     int pair_shape_ok;      // grid/method meet the paired kernel's shape conditions
     int any_shape_ok;       // ... or those of its form for any grid
     PSplit split_k;         // p-split of the tile kernels' stages that write k alone
+    PSplit split_scalar;    // ... and of the scalar kernel's stages without currents
 };
 
 #define CK(x)                                             \
@@ -349,6 +351,12 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
         }
         ctx->chunks_per_split = sp.chunks_per_split;
         ctx->nsplit = sp.nsplit;
+        // the stages that the scalar kernel takes on a grid of another one (df/dt
+        // alone, tau arrays) are cut for its own occupancy: a df/dt of 1000 x 200 FP64
+        // cells 30 us, by the line kernel's split 78 us; a step of 64^2 x 32^2 FP64
+        // cells with a tau array 463 us, by the tile kernel's 673 us
+        ctx->split_scalar = env ? sp : choose_psplit(nchunks, base_ctas, current_sm_count(),
+                                                     scalar_smem);
         // the stages of a run with fields that write k alone leave no partial
         // sums, so their split only has to fill the GPU (64^2 x 32^2 FP64: 128
         // CTAs in one wave instead of 256 in two)
@@ -376,12 +384,13 @@ int bolt_ctx_create(const BoltGrid* grid, const BoltParams* params, BoltCtx** ou
     for (int i = 0; i < nbuf && rc == BOLT_OK; ++i) rc = dev_alloc(ctx, &ctx->buf[i], fbytes);
     if (rc == BOLT_OK && p.fields_enabled) rc = dev_alloc(ctx, &ctx->kbuf, fbytes);
     const size_t plane = (size_t)g.N_q1 * g.N_q2 * g.N_s;
-    const int nsp = ctx->nsplit > 1 ? ctx->nsplit : 1;
+    const int nsp = std::max(std::max(ctx->nsplit, ctx->split_scalar.nsplit), 1);
     for (int i = 0; i < 2 && rc == BOLT_OK; ++i)
         rc = dev_alloc(ctx, (void**)&ctx->momP[i], (size_t)nsp * kNumMom * plane * sizeof(double));
     if (rc == BOLT_OK && p.fields_enabled) {
         const size_t fp = (size_t)ctx->Nq1g * ctx->Nq2g;
-        rc = dev_alloc(ctx, (void**)&ctx->jpart, (size_t)nsp * 3 * plane * sizeof(double));
+        rc = dev_alloc(ctx, (void**)&ctx->jpart,
+                       (size_t)std::max(ctx->nsplit, 1) * 3 * plane * sizeof(double));
         if (rc == BOLT_OK) rc = dev_alloc(ctx, (void**)&ctx->cell, 6 * fp * sizeof(double));
         if (rc == BOLT_OK) rc = dev_alloc(ctx, (void**)&ctx->yee, 6 * fp * sizeof(double));
         if (rc == BOLT_OK) rc = dev_alloc(ctx, (void**)&ctx->ebefore, 3 * fp * sizeof(double));
@@ -847,6 +856,7 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         const int n1 = ctx->ntiles1, n2 = ctx->ntiles2;
         const int inner = std::max(0, n1 - 2 * a.ext1) * std::max(0, n2 - 2 * a.ext2);
         const int count = region == 0 ? inner : n1 * n2 - inner;
+        ctx->q_nsplit = a.nsplit;
         if (count == 0) return BOLT_OK;
         grid.x = (unsigned)count;
     }
@@ -868,13 +878,19 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         a.chunks_per_split = ctx->split_k.chunks_per_split;
         grid.y = g.N_s * ctx->split_k.nsplit;
     }
+    // 1D1V: the line kernel, except for currents (q2 faces) and for
+    // bolt_dfdt without fields (as above)
+    const bool line = ctx->line_ok && !want_j && (!write_k || ctx->p.fields_enabled);
+    if (!line && !pair && !any && !want_j) {
+        a.nsplit = ctx->split_scalar.nsplit;
+        a.chunks_per_split = ctx->split_scalar.chunks_per_split;
+        grid.y = g.N_s * ctx->split_scalar.nsplit;
+    }
+    ctx->q_nsplit = a.nsplit;
     const size_t smem = pair || any ? qpair_smem(ctx->ntab, ctx->bgk, ctx->elem, any)
                                     : qstage_smem(ctx->tiling, ctx->elem, ctx->bgk,
                                                   ctx->bgk_direct, ctx->ntab);
     const int bgk = ctx->bgk, recon = ctx->recon_q;
-    // 1D1V: the line kernel, except for currents (q2 faces) and for
-    // bolt_dfdt without fields (as above)
-    const bool line = ctx->line_ok && !want_j && (!write_k || ctx->p.fields_enabled);
     cudaError_t e;
     if (line)
         e = ctx->elem == 4 ? launch_line_f32(a, recon, bgk, ctx->line, st)
@@ -1066,7 +1082,7 @@ static int ensure_state(BoltCtx* ctx, void* f, cudaStream_t st) {
     if ((ctx->bgk || electrostatic(ctx)) && ctx->mom_owner != f) {
         rc = launch_moments5(ctx, f, ctx->momP[ctx->cur_mom], st);
         if (rc) return rc;
-        ctx->cur_nsplit = 1;
+        ctx->mom_nsplit[ctx->cur_mom] = 1;
         ctx->mom_owner = f;
     }
     return rc;
@@ -1134,14 +1150,13 @@ static int run_rk_stage(BoltCtx* ctx, void* f, double dt, int k, cudaStream_t st
     const int dir = (ctx->p.bc_q1 != BOLT_BC_PERIODIC && ctx->p.bc_q1 != BOLT_BC_EXTERNAL) ||
                     (ctx->p.bc_q2 != BOLT_BC_PERIODIC && ctx->p.bc_q2 != BOLT_BC_EXTERNAL);
     const int fe = ctx->p.fields_enabled;
-    const int mo_split = fe ? 1 : ctx->nsplit;     // nsplit of partials written by a stage
-    double* m_in = ctx->momP[ctx->cur_mom ^ (k & 1)];
-    double* m_out = ctx->momP[ctx->cur_mom ^ (k & 1) ^ 1];
-    const int nin = k == 0 ? ctx->cur_nsplit : mo_split;
+    const int in = ctx->cur_mom ^ (k & 1);
+    double* m_in = ctx->momP[in];
+    double* m_out = ctx->momP[in ^ 1];
     StageIO io;
     memset(&io, 0, sizeof(io));
     io.mom_in = m_in;
-    io.nsplit_in = nin;
+    io.nsplit_in = ctx->mom_nsplit[in];
     // the moments of a stage's output serve the next one's Maxwellian, and its
     // electrostatic solve
     const bool track = ctx->bgk || electrostatic(ctx);
@@ -1175,7 +1190,10 @@ static int run_rk_stage(BoltCtx* ctx, void* f, double dt, int k, cudaStream_t st
         io.out1 = out1 = k == 0 ? A : f;
         peers_of(out1);
         ev = fe && !ctx->at_n;
-        if (region != 2) rc = run_stage(ctx, io, ev, dt, st, ev ? part : -1, region);
+        if (region != 2) {
+            rc = run_stage(ctx, io, ev, dt, st, ev ? part : -1, region);
+            ctx->mom_nsplit[in ^ 1] = fe ? 1 : ctx->q_nsplit;
+        }
         if (region == 0 || region == 1) return rc;
         if (fe && last_part) ctx->at_n ^= 1;
     } else {
@@ -1202,16 +1220,17 @@ static int run_rk_stage(BoltCtx* ctx, void* f, double dt, int k, cudaStream_t st
         io.out1 = out1 = stages[k].o1; io.base2 = stages[k].b2; io.c2 = stages[k].c2;
         io.out2 = stages[k].o2;
         peers_of(out1);
-        if (region != 2)
+        if (region != 2) {
             rc = run_stage(ctx, io, fe && stages[k].ev, dt, st, fe && stages[k].ev ? part : -1,
                            region);
+            ctx->mom_nsplit[in ^ 1] = fe ? 1 : ctx->q_nsplit;
+        }
         if (region == 0 || region == 1) return rc;
     }
     if (!last_part) return rc;
     if (!rc && dir) rc = launch_ghosts(ctx, out1, st);
     if (rc) return rc;
     if (last) {
-        ctx->cur_nsplit = mo_split;
         ctx->ghost_owner = f;
         ctx->mom_owner = track ? f : nullptr;
     }
@@ -1497,7 +1516,10 @@ static int dfdt_impl(BoltCtx* ctx, const void* f_dev, void* dfdt_dev, int evolve
                      double dt, int term, cudaStream_t st) {
     int rc = BOLT_OK;
     double* m = ctx->momP[ctx->cur_mom ^ 1];
-    if (ctx->bgk) rc = launch_moments5(ctx, f_dev, m, st);
+    if (ctx->bgk) {
+        rc = launch_moments5(ctx, f_dev, m, st);
+        ctx->mom_nsplit[ctx->cur_mom ^ 1] = 1;
+    }
     if (rc) return rc;
     StageIO io;
     memset(&io, 0, sizeof(io));

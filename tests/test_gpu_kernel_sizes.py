@@ -193,6 +193,30 @@ def test_infinite_collision_time(q, p, tau):
         assert bool(torch.isfinite(nls.f).all())
 
 
+@pytest.mark.parametrize('q,p', [((64, 64), (16, 16, 1)), ((21, 21), (33, 8, 1)),
+                                 ((1000, 1), (96, 1, 1))])
+@pytest.mark.parametrize('precision', ['fp64', 'fp32'])
+@pytest.mark.parametrize('integrator', ['RK2', 'RK4'])
+def test_kernels_take_turns(q, p, precision, integrator):
+    """Steps by the grid's own kernel and, with a tau array, by the scalar one, a
+    df/dt in between: each is cut for itself, so a stage may find another number of
+    partial moment sums than it leaves."""
+    spec = _spec(q, p, integrator=integrator, dt=1e-4)
+    nls = make_solver(spec, precision)
+    o = Oracle(spec, to_layout(nls.f, spec))
+    lib, ctx = nls._lib, nls._ctx
+    tau = torch.full_like(nls._fstore, spec['tau'])
+    for array in (False, True, True, False):
+        lib.bolt_set_tau_array(ctx, tau.data_ptr() if array else None)
+        nls.strang_timestep(spec['dt'])
+        o.step(spec['dt'])
+        out = torch.empty_like(nls._fstore)
+        assert lib.bolt_dfdt(ctx, nls._fstore.data_ptr(), out.data_ptr(), 0, 0.0, nls._stream()) == 0
+    nls.synchronize()
+    g = spec['N_ghost']
+    assert rel(interior(to_layout(nls.f, spec), g), interior(o.f, g)) < TOL[precision]
+
+
 @pytest.mark.parametrize('p', [(8, 6, 4), (7, 5, 3), (30, 1, 1)])
 @pytest.mark.parametrize('precision', ['fp64', 'fp32'])
 def test_semi_lagrangian_source_blocks(p, precision):
