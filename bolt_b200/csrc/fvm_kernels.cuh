@@ -582,16 +582,22 @@ struct PCellWalk {
     int i1, i2, i3;        // current p-cell
     int d1, d2, d3;        // the stride as (p1, p2, p3) steps
     int Np1, Np2;
-    __device__ __forceinline__ PCellWalk(int p, int stride, int np1, int np2)
-        : Np1(np1), Np2(np2) {
+    __device__ __forceinline__ PCellWalk(int p, int np1, int np2)
+        : d1(0), d2(0), d3(0), Np1(np1), Np2(np2) {
         i1 = p % np1;
         const int r = p / np1;
         i2 = r % np2;
         i3 = r / np2;
-        d1 = stride % np1;
-        const int rs = stride / np1;
-        d2 = rs % np2;
-        d3 = rs / np2;
+    }
+    __device__ __forceinline__ PCellWalk(int p, int stride, int np1, int np2)
+        : PCellWalk(p, np1, np2) {
+        set_stride(stride);
+    }
+    __device__ __forceinline__ void set_stride(int stride) {
+        d1 = stride % Np1;
+        const int rs = stride / Np1;
+        d2 = rs % Np2;
+        d3 = rs / Np2;
     }
     __device__ __forceinline__ void advance() {
         i1 += d1;
@@ -606,9 +612,12 @@ struct PCellWalk {
 
 // ---------------------------------------------------------------------------
 // moments (compute_moments.py:7-59 with moments.py:6-58), FP64 output.
-// One CTA per (ghosted q-cell, species).
+// One CTA per (ghosted q-cell, species).  STEPS: p-blocks of more than 256 cells, which
+// a thread steps through by a walker; its registers cost smaller ones two of six
+// CTAs per SM, and the divisions of its step more than the value (100^2 x 3 cells
+// 12 us, 21 us by the walker; 33 x 35 x 20^3 FP32 45 us by divisions, 29 us by it).
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool STEPS>
 __global__ void __launch_bounds__(256)
 moment_kernel(const T* f, int mid, double* out, int Ns, int Np1, int Np2, int Np3, int Nq1g,
               int Nq2g, SpeciesGrid sg) {
@@ -617,25 +626,30 @@ moment_kernel(const T* f, int mid, double* out, int Ns, int Np1, int Np2, int Np
     const int Np = Np1 * Np2 * Np3;
     const T* fp = f + ((long long)q * Ns + s) * Np;
     double acc = 0.0;
-    PCellWalk w(tid, 256, Np1, Np2);
-    for (int c = tid; c < Np; c += 256, w.advance()) {
-        const PVel V = lane_velocity(sg, s, w.i1, w.i2, w.i3);
-        const double fv = double(fp[c]);
-        double g;
-        switch (mid) {
-            case 0: g = fv; break;
-            case 1: g = fv * V.v1; break;
-            case 2: g = fv * V.v2; break;
-            case 3: g = fv * V.v3; break;
-            case 4: g = (0.5 * fv) * V.vsq; break;
-            case 5: g = (0.5 * fv) * (V.v1 * V.v1); break;
-            case 6: g = (0.5 * fv) * (V.v2 * V.v2); break;
-            case 7: g = (0.5 * fv) * (V.v3 * V.v3); break;
-            case 8: g = (fv * V.v1) * V.vsq; break;
-            case 9: g = (fv * V.v2) * V.vsq; break;
-            default: g = (fv * V.v3) * V.vsq; break;
+    if (tid < Np) {
+        PCellWalk w(tid, Np1, Np2);
+        if constexpr (STEPS) w.set_stride(256);
+        for (int c = tid; c < Np; c += 256) {
+            if (STEPS && c > tid) w.advance();
+            const PVel V = lane_velocity(sg, s, w.i1, w.i2, w.i3);
+            const double fv = double(fp[c]);
+            double g;
+            switch (mid) {
+                case 0: g = fv; break;
+                case 1: g = fv * V.v1; break;
+                case 2: g = fv * V.v2; break;
+                case 3: g = fv * V.v3; break;
+                case 4: g = (0.5 * fv) * V.vsq; break;
+                case 5: g = (0.5 * fv) * (V.v1 * V.v1); break;
+                case 6: g = (0.5 * fv) * (V.v2 * V.v2); break;
+                case 7: g = (0.5 * fv) * (V.v3 * V.v3); break;
+                case 8: g = (fv * V.v1) * V.vsq; break;
+                case 9: g = (fv * V.v2) * V.vsq; break;
+                default: g = (fv * V.v3) * V.vsq; break;
+            }
+            acc += g;
+            if constexpr (!STEPS) break;
         }
-        acc += g;
     }
     acc = warp_sum(acc);
     if ((tid & 31) == 0) red[tid >> 5] = acc;

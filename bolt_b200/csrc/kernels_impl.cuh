@@ -118,8 +118,9 @@ cudaError_t BOLT_CAT(launch_moment_, BOLT_SUFFIX)(const void* f, int mid, double
                                                   int Np1, int Np2, int Np3, int Nq1g, int Nq2g,
                                                   const SpeciesGrid& sg, cudaStream_t st) {
     dim3 grid(Nq1g * Nq2g, Ns);
-    moment_kernel<BOLT_T><<<grid, 256, 0, st>>>(static_cast<const BOLT_T*>(f), mid, out, Ns, Np1,
-                                                Np2, Np3, Nq1g, Nq2g, sg);
+    auto k = Np1 * Np2 * Np3 > 256 ? moment_kernel<BOLT_T, true> : moment_kernel<BOLT_T, false>;
+    k<<<grid, 256, 0, st>>>(static_cast<const BOLT_T*>(f), mid, out, Ns, Np1,
+                             Np2, Np3, Nq1g, Nq2g, sg);
     return cudaGetLastError();
 }
 
