@@ -20,10 +20,11 @@ constexpr int kFieldCluster = 8, kFieldThreads = 1024;
 constexpr int kFieldClusterCells = 1 << 14;
 
 // all threads of the cluster, their global memory accesses before it visible
-// after it
+// after it (not the .aligned form: the passes before it end in loops whose threads
+// leave at different times)
 __device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\t"
+                 "barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 __device__ __forceinline__ int wrapi(int x, int n) { return ((x % n) + n) % n; }

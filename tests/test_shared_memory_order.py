@@ -1,6 +1,7 @@
-"""Shared memory that one thread writes and another one reads needs a CTA barrier
-in between; where a missing one would show only once in many runs, the order in
-the source is checked."""
+"""Barriers whose absence or misuse would show only once in many runs, if ever: the
+source is checked for them.  Shared memory that one thread writes and another one
+reads needs a CTA barrier in between, and a barrier of the .aligned form needs a
+converged warp."""
 
 import os
 import re
@@ -26,3 +27,14 @@ def test_currents_are_zeroed_before_a_barrier():
     prologue = src[src.index('void qpair_prologue('):]
     body = prologue[:re.search(r'\n}', prologue).start()]
     assert body.rstrip().endswith('__syncthreads();')
+
+
+def test_cluster_barrier_takes_diverged_warps():
+    """Between the passes of the field update, whose loops the threads of a warp leave
+    at different times."""
+    src = _source('fdtd_kernels.cuh')
+    barrier = src[src.index('void cluster_barrier()'):]
+    barrier = barrier[:barrier.index('}')]
+    assert 'barrier.cluster.arrive.release;' in barrier
+    assert 'barrier.cluster.wait.acquire;' in barrier
+    assert '.aligned' not in barrier
