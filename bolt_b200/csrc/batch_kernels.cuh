@@ -24,7 +24,7 @@
 //     out1 accumulated per thread across chunks, non-finite check.
 //
 // What bounds it: instruction issue and the latency of the loads (the working
-// set of the 256-run sweep fits L2): 81 us per stage of 10.9M cells (99 us with
+// set of the 256-run sweep fits L2): 82 us per stage of 10.9M cells (99 us with
 // the three-weight faces and the reduction of the exponent in v - u).  Eight
 // cells per warp as f32x2 pairs gave 86 us, and the same without shared memory
 // 90 us and up to 30 % more on batches of tens of runs.
@@ -86,8 +86,8 @@ __device__ __forceinline__ float batch_exp2(double x) {
 // Maxwellian parameters of one q-cell from its raw moment sums
 // (collision_operator.py:102-118, f0 :49-65 with p_dim = 1):
 // {n A, c0, c1, c2} with f0(v) = n A 2^(c0 + c1 v + c2 v^2), the exponent
-// -m (v - u1)^2 / (2 kB T) expanded in v (FP64: its terms cancel to ~1e-13 at
-// the widest grids, against 2^-22 of the exponential)
+// -m (v - u1)^2 / (2 kB T) expanded in v (FP64: its terms cancel to 2^-53 m u1^2 /
+// (kB T), the relative error that T itself has from the moments' difference)
 __device__ __forceinline__ void batch_maxwell(const BatchRunDev& R, const double* mm,
                                               double* out) {
     const double eps = 1e-30;

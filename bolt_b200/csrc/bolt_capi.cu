@@ -208,8 +208,10 @@ static const CUtensorMap* get_tmap(BoltCtx* ctx, const void* ptr, int kind) {
 // (fft.py:9-78 with one q2 cell): E = real(ifft(-i rho_hat / (2 pi k))), k = 0 left
 // out, is sum_j G_{i-j} rho_j with G_m = (1/n) sum_{k=1}^{(n-1)/2} sin(2 pi k m / n)
 // / (pi k / (n dq)); the Nyquist mode of an even n is imaginary and drops out.
-// Up to kGreenMax cells: every p-stage CTA reads n of its values (16 KB), which
-// costs less than the solve's launches; longer lines use the FFT.
+// Up to kGreenMax cells: every p-stage CTA reads n of its values (16 KB) and the
+// line's densities, which grows with n^2, while the solve's launches cost the same.
+// RK2 step of n x 256 FP64 cells, by the FFT and here: 512 127 and 45 us, 1024 136 and
+// 57 us, 2048 205 and 143 us (FP32 131 and 78 us).
 constexpr int kGreenMax = 2048;
 
 static std::vector<double> line_green(int n, double dq) {
@@ -817,12 +819,18 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
     a.full_chunks = (ctx->Np % PW) == 0;
     a.sg = ctx->sg;
     dim3 grid(ctx->ntiles1 * ctx->ntiles2, g.N_s * ctx->nsplit);
-    // the paired kernel covers the fused 2-D stage with every buffer reachable
-    // by TMA; everything else (1-D tilings, write-k mode, currents, tau arrays,
-    // sizes off its tiles) runs the scalar kernel
-    // (so do the write-k stages of field-coupled steps, unless they also
-    // accumulate currents; bolt_dfdt without fields keeps the scalar kernel,
-    // the one bolt_dfdt_noalloc runs, so the two agree to the bit)
+    // Which kernel:
+    //   line    1D1V grids that line_fits takes (periodic q2, one p2 and p3 cell)
+    //   pair    2-D stages on whole 8x8 tiles and chunks of p, every buffer
+    //           reachable by TMA: FP32, FP64 in its throughput form and in the
+    //           reference's order
+    //   any     the same kernel on every other 2-D grid with three ghost cells and
+    //           one periodic image per cell, and for the stages that accumulate
+    //           currents
+    //   scalar  the rest: tau arrays, fewer ghost cells, tiny q-grids, tables too
+    //           large for a CTA, one q2 cell with p2 or p3, FP32 currents of several
+    //           species, and bolt_dfdt without fields (the kernel that
+    //           bolt_dfdt_noalloc runs, so the two agree to the bit)
     bool tiles = ctx->pair_enabled &&
                  (write_k ? ctx->p.fields_enabled != 0 : a.base1 != nullptr) &&
                  ctx->tau_arr == nullptr;
@@ -860,9 +868,7 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         if (count == 0) return BOLT_OK;
         grid.x = (unsigned)count;
     }
-    // sizes off the tiles, and the stages that accumulate currents: the same
-    // kernel for any grid (its loads by TMA where rows and base are aligned).
-    // FP32 runs with fields and several species keep the scalar kernel there: a
+    // any: loads by TMA where rows and base are aligned.  FP32 runs with fields and several species keep the scalar kernel there: a
     // neutral plasma's current is the difference of nearly equal species
     // currents, at the level of their FP32 rounding, so another rounding of the
     // faces would be another electric field (FP64 has the same bits either way)
@@ -878,8 +884,7 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         a.chunks_per_split = ctx->split_k.chunks_per_split;
         grid.y = g.N_s * ctx->split_k.nsplit;
     }
-    // 1D1V: the line kernel, except for currents (q2 faces) and for
-    // bolt_dfdt without fields (as above)
+    // (currents need the q2 faces, which the line kernel leaves out)
     const bool line = ctx->line_ok && !want_j && (!write_k || ctx->p.fields_enabled);
     if (!line && !pair && !any && !want_j) {
         a.nsplit = ctx->split_scalar.nsplit;

@@ -1,7 +1,7 @@
 // FP64 stage kernel in the reference's operation order on 8x8 tiles: the fused
 // RK stage of qpair_kernel.cuh, built with -fmad=false so that no multiply-add
 // is contracted.  Same bits per value as the scalar stage kernel of
-// kernels_f64.cu, which takes every other grid.
+// kernels_f64.cu; grids off the tiles run the forms of kernels_f64exactany.cu.
 #include "launch.h"
 #include "qpair_kernel.cuh"
 

@@ -137,7 +137,9 @@ struct PShape {
 // side by side (seg counts the pairs).  The shape minimises thread-time
 // of a CTA, scaled up while the SM holds fewer than 24 warps of this launch
 // (latency not hidden): 2D blocks take the fewest threads that still fill the
-// SM, small q-grids take as many threads as shorten the walk.
+// SM, small q-grids take as many threads as shorten the walk.  The three cells, the 24
+// warps and the 1.5 per value are a model; registers, which admit fewer CTAs than
+// shared memory does (64 each: two of 416 threads, not three), are not in it.
 inline PShape choose_pshape(int n1, int n2, int n3, size_t elem, bool pairs, long long ctas,
                             int sms) {
     const int n[3] = {n1, n2, n3};

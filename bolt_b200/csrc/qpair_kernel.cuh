@@ -48,8 +48,8 @@
 // goes from the q2 walkers' registers to memory.  The scalar kernel (8 warps,
 // four divisions a face, single-buffered halo) left the FP64 pipe idle most of
 // the time: an RK4 step of 64^2 x 24^3 cells took 9.62 ms, here 3.59 ms (its
-// bytes alone 1.2 ms; 3.78 ms with the q1 walk rolled); what bounds it now is the
-// latency of the dependent FP64 chains at 16 warps per SM.
+// bytes alone 1.2 ms; 3.78 ms with the q1 walk rolled).  What bounds it now: the FP64
+// pipe, busy 62 % of cycles, and the latency of its dependent chains at 16 warps per SM.
 //
 // QG_ANY, QG_CURRENTS: any grid.  The halo and base tiles come by TMA where rows
 // are multiples of 16 bytes (cells outside the array read as zero), else by
@@ -57,16 +57,22 @@
 // outputs go from the q2 walkers' registers to memory under a mask, and the
 // accumulator's increment by one red.global.add per element.  An RK2 step of
 // 75 x 50 x 45 x 35 FP32 cells between mirrors (rows of 6300 bytes, by copies)
-// took 551 us on the scalar kernel, here 150 us (180 us while an out2 tile that
-// FP32 does not need there left room for one CTA per SM).  The currents add up
+// took 551 us on the scalar kernel, here 152 us (180 us while an out2 tile that
+// FP32 does not need there left room for one CTA per SM; 150 us with faces that a
+// jump beyond 3e4 beside uniform data overflows).  The FP32 forms' tables and products
+// of the Maxwellian are FP32, where the scalar kernel's are FP64: no larger error while
+// dt is a small part of tau, up to 2.5 times at dt = tau.  The currents add up
 // eight cells at a time over the warp: a currents stage of 64^2 x 32^2 FP32 cells
 // went from 78 us to 37 us, and with nine exchanges instead of forty to 29 us
 // (FP64: from 106 us to 82 us).
 //
-// Launch conditions (checked by the host): FP32 or FP64, any reconstruction in q, 8x8 tiling,
-// N_q1, N_q2 multiples of 8 and at least 2 N_g, N_p multiple of 32, N_p1
-// multiple of 8, BGK by exp tables, all five buffers 16-byte aligned, f with
-// fewer than 2^31 elements (32-bit offsets).
+// Launch conditions (checked by the host), every form: a 2-D tiling, N_q1 and N_q2 at
+// least 2 N_g, BGK by exp tables that fit a CTA, no tau array, f with fewer than 2^31
+// elements (32-bit offsets).
+//   QG_TILES     N_q1, N_q2 multiples of 8, N_p of 32 and N_p1 of 8, all buffers
+//                reachable by TMA (16-byte aligned, N_g >= 3)
+//   QG_ANY       N_g >= 3, buffers at any alignment of their type
+//   QG_CURRENTS  as QG_ANY, the k-only stage of a run with fields
 #pragma once
 
 #include <type_traits>

@@ -406,9 +406,9 @@ int  bolt_set_timing(BoltCtx* ctx, int on);
 int  bolt_timings(BoltCtx* ctx, double* ms_out);
 
 /* Number of kernels launched through this context so far, and how many of
- * them were the paired stage kernel (the fused q-stage taken for FP32 and
- * BOLT_F64_FAST 8x8-tiled grids; every other stage runs the
- * one-cell-per-thread kernel).
+ * them were the paired stage kernel (the q-stage on whole 8x8 tiles and chunks,
+ * FP32 and both FP64 forms; other grids run its form for any grid, the 1D1V
+ * kernel or the one-cell-per-thread kernel).
  * Diagnostics: the reference has no counterpart. */
 long long bolt_launch_count(BoltCtx* ctx);
 long long bolt_paired_launch_count(BoltCtx* ctx);
