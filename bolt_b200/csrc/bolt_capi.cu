@@ -828,9 +828,10 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
     //           one periodic image per cell, and for the stages that accumulate
     //           currents
     //   scalar  the rest: tau arrays, fewer ghost cells, tiny q-grids, tables too
-    //           large for a CTA, one q2 cell with p2 or p3, FP32 currents of several
-    //           species, and bolt_dfdt without fields (the kernel that
-    //           bolt_dfdt_noalloc runs, so the two agree to the bit)
+    //           large for a CTA, one q2 cell with p2 or p3, off the tiles in FP32
+    //           currents of several species and steps beyond 0.07 tau, and
+    //           bolt_dfdt without fields (the kernel that bolt_dfdt_noalloc runs, so
+    //           the two agree to the bit)
     bool tiles = ctx->pair_enabled &&
                  (write_k ? ctx->p.fields_enabled != 0 : a.base1 != nullptr) &&
                  ctx->tau_arr == nullptr;
@@ -868,11 +869,20 @@ static int launch_qstage(BoltCtx* ctx, const StageIO& io, int write_k, int want_
         if (count == 0) return BOLT_OK;
         grid.x = (unsigned)count;
     }
-    // any: loads by TMA where rows and base are aligned.  FP32 runs with fields and several species keep the scalar kernel there: a
-    // neutral plasma's current is the difference of nearly equal species
-    // currents, at the level of their FP32 rounding, so another rounding of the
-    // faces would be another electric field (FP64 has the same bits either way)
-    const bool any = tiles && !pair && ctx->any_shape_ok &&
+    // any: loads by TMA where rows and base are aligned.  FP32 runs with fields and
+    // several species keep the scalar kernel there: a neutral plasma's current is
+    // the difference of nearly equal species currents, at the level of their FP32
+    // rounding, so another rounding of the faces would be another electric field
+    // (FP64 has the same bits either way).
+    // Its FP32 form also has the Maxwellian's factors in FP32, where the scalar
+    // kernel's are FP64: their rounding shows where a stage replaces much of f by
+    // it.  11 x 13 x 15 x 13 x 14 cells, f from 64 bits after ten RK2 steps by FP64 and
+    // FP32 factors: 7.1e-8 each at dt = 0.02 tau, 5.7e-8 and 5.9e-8 at 0.1 tau, 5.6e-8
+    // and 11e-8 at tau.  So beyond 0.07 tau the scalar kernel stays, as for a df/dt
+    // whose step is not known.
+    const bool stiff = ctx->elem == 4 && ctx->bgk &&
+                       !(io.base1 && std::fabs(io.c1) <= 0.07 * std::fabs(ctx->p.tau));
+    const bool any = tiles && !pair && ctx->any_shape_ok && !stiff &&
                      !(ctx->elem == 4 && ctx->p.fields_enabled && g.N_s > 1);
     if (any && a.use_tma && a.base1) {
         const CUtensorMap* m = (uintptr_t)a.base1 % 16 == 0

@@ -59,9 +59,9 @@
 // 75 x 50 x 45 x 35 FP32 cells between mirrors (rows of 6300 bytes, by copies)
 // took 551 us on the scalar kernel, here 152 us (180 us while an out2 tile that
 // FP32 does not need there left room for one CTA per SM; 150 us with faces that a
-// jump beyond 3e4 beside uniform data overflows).  The FP32 forms' tables and products
-// of the Maxwellian are FP32, where the scalar kernel's are FP64: no larger error while
-// dt is a small part of tau, up to 2.5 times at dt = tau.  The currents add up
+// jump beyond 3e4 beside uniform data overflows).  The FP32 form's
+// Maxwellian tables and their products are FP32, where the scalar kernel's are FP64; the
+// host keeps it to steps of at most 0.07 tau, where that does not show.  The currents add up
 // eight cells at a time over the warp: a currents stage of 64^2 x 32^2 FP32 cells
 // went from 78 us to 37 us, and with nine exchanges instead of forty to 29 us
 // (FP64: from 106 us to 82 us).

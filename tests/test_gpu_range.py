@@ -1,5 +1,6 @@
 """States far from the smooth, order-one ones of the other tests: jumps of large
-values beside exactly uniform data, and values whose squares leave the range."""
+values beside exactly uniform data, values whose squares leave the range, and steps as
+long as the collision time."""
 
 import os
 import sys
@@ -158,3 +159,18 @@ def test_reference_order_beside_a_huge_value(monkeypatch, kernel, top):
         return
     assert small.sum() > 0.5 * want.size
     assert rel(got[small], want[small]) < TOL['fp64']
+
+
+@pytest.mark.parametrize('q,p', [((11, 13), (15, 13, 14)), ((9, 10), (20, 18, 1)), ((20, 1), (60, 1, 1))])
+@pytest.mark.parametrize('fields', [False, True])
+def test_stiff_source(q, p, fields):
+    """dt = tau in FP32, off the whole tiles: RK2 keeps half of f's error and adds the
+    rounding of two stored stages (3.4e-8 rms each), 5.5e-8 in all at worst; a Maxwellian
+    of rounded factors would double that after ten steps."""
+    kw = dict(fields_enabled=True, fields_type='electrostatic', fields_solver='fft',
+              charge=[-0.1]) if fields else {}
+    spec = _spec(q, p, dt=1e-3, tau=1e-3, steps=30, **kw)
+    nls = make_solver(spec, 'fp32')
+    o = Oracle(spec, to_layout(nls.f, spec))
+    got, want = _steps(nls, o, spec)
+    assert rel(got, want) < 1e-7
