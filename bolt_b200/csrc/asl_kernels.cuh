@@ -492,7 +492,7 @@ __device__ __forceinline__ bool asl_source_cell(const QStageArgs& a, const T* fi
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) asl_source_kernel(const QStageArgs a, const void* in,
                                                             void* out, double dt, int* flag) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double qq[5], mom[kNumMom];
     __shared__ double red[8][kNumMom];
     const int ntab = a.Np1 + a.Np2 + a.Np3, tid = threadIdx.x;

@@ -38,3 +38,13 @@ def test_cluster_barrier_takes_diverged_warps():
     assert 'barrier.cluster.arrive.release;' in barrier
     assert 'barrier.cluster.wait.acquire;' in barrier
     assert '.aligned' not in barrier
+
+
+def test_dynamic_shared_memory_has_one_alignment():
+    """The kernels of a translation unit share the declaration: TMA's destinations in
+    one of them need the 128 bytes that another one must not take back."""
+    found = []
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith(('.cuh', '.cu', '.h')):
+            found += re.findall(r'extern\s+__shared__\s+__align__\((\d+)\)[^;]*;', _source(name))
+    assert len(found) >= 4 and set(found) == {'128'}
